@@ -982,36 +982,75 @@ __device__ __forceinline__ int pair_eval(V3<double> xi, V3<double> xj, V3<double
     const V3<double> Dv = xj - xi;
     const double d2 = dot(Dv, Dv);
     const double s = (double)ri + (double)rj;
-    Real delta;
-    V3<Real> nn;
-    if constexpr (sizeof(Real) == 4) {
-        // the overlap's numerator s^2 - d^2 in FP64 (no cancellation), the
-        // rest in FP32: delta = (s^2 - d^2) / (s + d), n = D / d
-        const float d2f = (float)d2;
-        const float dist = sqrtf(d2f);
-        delta = (float)(s * s - d2) / ((float)s + dist);
-        if (!(delta > 0.f && d2f > 0.f)) {
-            h = zero3<double>();
-            return 0;
+    Real delta, rstar, mstar;
+    V3<Real> nn, Ft, Mr;
+    V3<double> hn = h;
+    const V3<Real> dd = cvt<Real>(dj - di), w = ri * ai + rj * aj, Wr = ai - aj;
+    bool ok = false;
+    if (pp.fast) {   // the ordinary case, with the branch-free quotients and roots
+        if constexpr (sizeof(Real) == 4) {
+            // the overlap's numerator s^2 - d^2 in FP64 (no cancellation), the
+            // rest in FP32: delta = (s^2 - d^2) / (s + d), n = D / d
+            const float num = (float)(s * s - d2);
+            if (!(num > 0.f)) {
+                h = zero3<double>();
+                return 0;
+            }
+            const float d2f = (float)d2;
+            const float dist = x_sqrt(d2f);
+            delta = x_div(num, (float)s + dist);
+            const float inv = x_rcp(dist);
+            nn = mk((float)Dv.x * inv, (float)Dv.y * inv, (float)Dv.z * inv);
+            ok = x_in(d2f) && x_in(num);
+        } else {
+            if (!(d2 < s * s * 1.0000001)) {   // d >= s beyond any rounding (or not a number)
+                h = zero3<double>();
+                return 0;
+            }
+            const double dist = x_sqrt(d2);
+            delta = s - dist;
+            ok = x_in(d2);
+            if (ok && !(delta > 0.0)) {
+                h = zero3<double>();
+                return 0;
+            }
+            nn = Dv * x_rcp(dist);
         }
-        const float inv = 1.f / dist;
-        nn = mk((float)Dv.x * inv, (float)Dv.y * inv, (float)Dv.z * inv);
-    } else {
-        const double dist = sqrt(d2);
-        delta = (Real)(s - dist);
-        if (!(delta > (Real)0 && dist > 0.0)) {
-            h = zero3<double>();
-            return 0;
-        }
-        const double inv = 1.0 / dist;
-        nn = cvt<Real>(Dv * inv);
+        const Real mi = density * (Real)8 * ri * ri * ri, mj = density * (Real)8 * rj * rj * rj;
+        const Real rr = ri * rj, mm = mi * mj;
+        rstar = x_div(rr, ri + rj);
+        mstar = x_div(mm, mi + mj);
+        ok = ok && x_in(rr) && x_in(mm);
+        ok = contact_law_fast<Real>(delta, nn, rstar, mstar, dd - cross(w, nn), Wr, hn, inv_dt, pp, Fi, Ft, Mr) && ok;
     }
-    const Real rstar = ri * rj / (ri + rj);
-    const Real mi = density * (Real)8 * ri * ri * ri, mj = density * (Real)8 * rj * rj * rj;
-    const Real mstar = mi * mj / (mi + mj);
-    const V3<Real> U = cvt<Real>(dj - di) - cross(ri * ai + rj * aj, nn);
-    V3<Real> Ft, Mr;
-    contact_law<Real>(delta, nn, rstar, mstar, U, ai - aj, h, inv_dt, pp, Fi, Ft, Mr);
+    if (!ok) {   // the whole range, with the library's
+        if constexpr (sizeof(Real) == 4) {
+            const float d2f = (float)d2;
+            const float dist = sqrtf(d2f);
+            delta = (float)(s * s - d2) / ((float)s + dist);
+            if (!(delta > 0.f && d2f > 0.f)) {
+                h = zero3<double>();
+                return 0;
+            }
+            const float inv = 1.f / dist;
+            nn = mk((float)Dv.x * inv, (float)Dv.y * inv, (float)Dv.z * inv);
+        } else {
+            const double dist = sqrt(d2);
+            delta = (Real)(s - dist);
+            if (!(delta > (Real)0 && dist > 0.0)) {
+                h = zero3<double>();
+                return 0;
+            }
+            const double inv = 1.0 / dist;
+            nn = cvt<Real>(Dv * inv);
+        }
+        rstar = ri * rj / (ri + rj);
+        const Real mi = density * (Real)8 * ri * ri * ri, mj = density * (Real)8 * rj * rj * rj;
+        mstar = mi * mj / (mi + mj);
+        hn = h;
+        contact_law<Real>(delta, nn, rstar, mstar, dd - cross(w, nn), Wr, hn, inv_dt, pp, Fi, Ft, Mr);
+    }
+    h = hn;
     const V3<Real> nxf = cross(nn, Ft);
     Ti = ri * nxf + Mr;
     Tj = rj * nxf - Mr;
