@@ -966,7 +966,9 @@ int recompute_segment(dem_ctx* c, long long every) {
     int rc;
     for (long long t = 0; t < every; t += K) {
         c->carry = w->lists[t / K].carry;
+        c->window_follows = use_batches(c);
         rc = relist(c, c->cur);
+        c->window_follows = false;
         c->carry = nullptr;
         if (rc) return rc;
         c->cur = 1 - c->cur;

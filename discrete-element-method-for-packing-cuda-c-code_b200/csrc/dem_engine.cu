@@ -178,6 +178,11 @@ __global__ void k_pour_activate(long long nold, long long nnew, const PRec<Real>
 }
 
 // --------------------------------------------------------------- re-list
+// Outside a graph the outer build's kernels are launched at every re-list and
+// those that do the work leave at once when the check found the list still
+// valid (need: its word; null in a graph, where a conditional node holds them).
+__device__ __forceinline__ bool build_off(const uint* need) { return need && *need == 0u; }
+
 // Scatter each particle (id, cell, list coordinates x,y,z,r in the list
 // precision) into its cell's range at its arrival slot, unordered inside the
 // cell, and record each particle's slot (tpos); the count array returns to
@@ -188,9 +193,8 @@ template <typename Real>
 __global__ void k_scatter(long long n, const uint* __restrict__ key, const uint* __restrict__ arrival,
                           const uint* __restrict__ cstart, uint* __restrict__ count, const PRec<Real>* __restrict__ S,
                           const Real* __restrict__ R, GridC g, uint* __restrict__ sidu, uint* __restrict__ skeyu,
-                          R4<Real>* __restrict__ sposu, uint* __restrict__ tpos) {
-    pdl_wait();
-    pdl_trigger();
+                          R4<Real>* __restrict__ sposu, uint* __restrict__ tpos, const uint* __restrict__ need) {
+    if (build_off(need)) return;
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint c = key[i];
@@ -222,7 +226,8 @@ constexpr uint kScr = 8;
 // oskin then (with room for the rounding of the FP32 tests), so filtering the
 // outer rows with the exact candidate test gives exactly the pairs the cell
 // walk would give.  In a window graph the build is the body of a conditional
-// node that the check kernel switches on; an eager re-list always builds.
+// node that the check kernel switches on; an eager re-list launches its
+// kernels, which leave at once while the list is valid (build_off).
 
 // A particle's list coordinates (as k_scatter writes them): position relative
 // to the grid origin and radius, in the list precision.
@@ -250,7 +255,7 @@ constexpr uint kNearWall = 0x80000000u;
 template <typename Real>
 __global__ void k_outer_check(long long n, const PRec<Real>* __restrict__ S, const Real* __restrict__ R, GridC g,
                               double hx, double hy, double half_skin, uint* __restrict__ ikey, Planes3<double> xo,
-                              double odelta2, const uint* __restrict__ oflag, uint* __restrict__ wcount, int cond,
+                              double odelta2, uint* oflag, uint* __restrict__ wcount, int cond,
                               cudaGraphConditionalHandle h) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) *wcount = 0u;   // the candidate pass counts the wall candidates
@@ -268,7 +273,10 @@ __global__ void k_outer_check(long long n, const PRec<Real>* __restrict__ S, con
         const int cz = cell_axis<Real>(p.z, g.oz, csr, g.gz, xl);
         ikey[i] = (((uint)cz * (uint)g.gy + (uint)cy) * (uint)g.gx + (uint)cx) | (near ? kNearWall : 0u);
     }
-    if (cond && __any_sync(0xffffffffu, need) && lane_id() == 0) cudaGraphSetConditional(h, 1u);
+    if (__any_sync(0xffffffffu, need) && lane_id() == 0) {
+        if (cond) cudaGraphSetConditional(h, 1u);
+        else oflag[1] = 1u;   // outside a graph: the build's kernels read it (build_off)
+    }
 }
 
 // Cell key of each particle on the outer grid (calcHashD's role,
@@ -276,7 +284,8 @@ __global__ void k_outer_check(long long n, const PRec<Real>* __restrict__ S, con
 // sort of k_scatter).
 template <typename Real>
 __global__ void k_cell_hash(long long n, const PRec<Real>* __restrict__ S, GridC g, uint* __restrict__ key,
-                            uint* __restrict__ count, uint* __restrict__ arrival) {
+                            uint* __restrict__ count, uint* __restrict__ arrival, const uint* __restrict__ need) {
+    if (build_off(need)) return;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const V3<double> p = ld_pos<false>(S + i);
@@ -322,7 +331,8 @@ __device__ __forceinline__ uint walk27_all(long long t, const R4<Real>& me, uint
 template <typename Real>
 __global__ void k_outer_count(long long n, const uint* __restrict__ sid2, const R4<Real>* __restrict__ spos,
                               const uint* __restrict__ skey, const uint* __restrict__ cstart, GridC g, Real oskin,
-                              uint* __restrict__ ocnt) {
+                              uint* __restrict__ ocnt, const uint* __restrict__ need) {
+    if (build_off(need)) return;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     ocnt[sid2[t]] = walk27_all<Real, false>(t, spos[t], skey[t], g, cstart, sid2, spos, oskin, nullptr, 0);
@@ -336,7 +346,8 @@ __global__ void k_outer_fill(long long n, const uint* __restrict__ sid2, const R
                              const uint* __restrict__ skey, const uint* __restrict__ cstart, GridC g, Real oskin,
                              const uint* __restrict__ coff, uint* __restrict__ cln, long long ccap,
                              const PRec<Real>* __restrict__ S, Planes3<double> xo, uint* __restrict__ oflag,
-                             EngineWords* words) {
+                             EngineWords* words, const uint* __restrict__ need) {
+    if (build_off(need)) return;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool over = (long long)coff[n] > ccap;
     if (t == 0) {
@@ -470,6 +481,12 @@ __device__ __forceinline__ FilterCounts<K> filter_items(long long i0, DEM_FILTER
 // and the kind above (1: the tile's own total, 2: the total through the
 // tile); the fill clears them for the next re-list.
 constexpr int kFilterThreads = 512, kFilterItems = 4, kFilterTile = kFilterThreads * kFilterItems;
+// limits and words of the bounded waits (grid_wait, tile_wait)
+constexpr unsigned long long kBarrierNs = 1000000000ull;   // 1 s
+constexpr uint kBarrierMinPolls = 200000u;                 // >= ~0.1 s of polling
+constexpr uint kBarrierMaxPolls = 20000000u;               // a few seconds at most
+constexpr int kBarGiveUp = 32;                             // bar[32]: own 128-byte line
+constexpr int kBarWords = 64;                              // words zeroed per launch
 constexpr int kCcThreads = 256;   // the component pass: one bound-list entry per thread and tile
 constexpr unsigned long long kLbAgg = 1ull << 32, kLbIncl = 2ull << 32;
 constexpr int kLbSpin = 1 << 16;   // a look-back word not published after this many polls: kStBarrier
@@ -812,7 +829,8 @@ __global__ void __launch_bounds__(kCcThreads)
               const uint* __restrict__ off, const uint* __restrict__ bpos, const uint* __restrict__ blist,
               const uint* __restrict__ parent, const uint* __restrict__ size, const uint* __restrict__ pairs,
               uint* base, uint* __restrict__ fill, uint* __restrict__ order, uint* bw, uint* __restrict__ batch,
-              uint* ccw, uint* __restrict__ cc_skip, uint* lbc, EngineWords* words) {
+              uint* ccw, uint* __restrict__ cc_skip, uint* lbc, EngineWords* words, uint* bar, int cond,
+              cudaGraphConditionalHandle hw) {
     constexpr int W = kCcThreads / 32;
     __shared__ uint s_tile, s_last, s_agg, s_pre;
     __shared__ uint s_w[W], s_red[W];
@@ -961,10 +979,14 @@ __global__ void __launch_bounds__(kCcThreads)
         if (skip) *cc_skip = skip - 1u;
         else if (maxc > P) *cc_skip = kDenseSkip;   // a component larger than a block (a dense bed)
     }
-    if (!run || __ldcg(ccw + 1)) return;
-    const uint nbatch = (nb + tgt - 1) / tgt;
-    const uint bmax = (long long)nbatch < nbmax ? nbatch : (uint)nbmax;
-    for (uint b = me; b <= bmax; b += blockDim.x) cc_batch_entry(b, nb, tgt, nbmax, nbb, P, Q, bw, batch, ccw);
+    if (run && !__ldcg(ccw + 1)) {
+        const uint nbatch = (nb + tgt - 1) / tgt;
+        const uint bmax = (long long)nbatch < nbmax ? nbatch : (uint)nbmax;
+        for (uint b = me; b <= bmax; b += blockDim.x) cc_batch_entry(b, nb, tgt, nbmax, nbb, P, Q, bw, batch, ccw);
+    }
+    if (me < (uint)(2 * kBarWords)) bar[me] = 0u;   // the wait words of the kernels that follow
+    __syncthreads();
+    if (cond && me == 0 && __ldcg(ccw + 1)) cudaGraphSetConditional(hw, 1u);   // the tiles' node
 }
 
 // ------------------------------------------------------------ pair force
@@ -1057,6 +1079,16 @@ __device__ __forceinline__ int pair_eval(V3<double> xi, V3<double> xj, V3<double
     return 1;
 }
 
+// Words of the tile path (k_tile): [0] particles per tile, [1] tiles, [2]
+// nonzero: a tile does not fit (the grid-barrier window kernel has the
+// window), [3] windows since the curve was computed, [4] nonzero: the curve
+// is valid, [5] bytes of a stage in shared memory, [6] sixteenths the tiles
+// are smaller because one did not fit, [7] nonzero: this window computes the
+// curve.
+enum : uint {
+    kTwP = 0, kTwTiles = 1, kTwOver = 2, kTwAge = 3, kTwValid = 4, kTwStage = 5, kTwShrink = 6, kTwNeed = 7, kTwWords = 8
+};
+
 // Arguments of the PCCP step kernels (pair items, bound particles, free
 // particles) and of the window kernel that runs all of a window's steps.
 template <typename Real> struct StepArgs {
@@ -1076,6 +1108,7 @@ template <typename Real> struct StepArgs {
     // set, in which case the grid-barrier window kernel steps the window
     int batch;
     const uint* ccw;
+    const uint* tw;               // tile path's words (nullptr: no tiles)
     EngineWords* words;
     double *dbgF, *dbgT;
     uint* dbgC;
@@ -1517,12 +1550,6 @@ __global__ void __launch_bounds__(256) k_free_run(StepArgs<Real> a, int slot0, i
 // if it steps backwards, and the poll floor keeps a forward step of the timer
 // (the driver recalibrates %globaltimer) from ending a healthy wait.  A later
 // launch starts with its own give-up word clear.
-constexpr unsigned long long kBarrierNs = 1000000000ull;   // 1 s
-constexpr uint kBarrierMinPolls = 200000u;                 // >= ~0.1 s of polling
-constexpr uint kBarrierMaxPolls = 20000000u;               // a few seconds at most
-constexpr int kBarGiveUp = 32;                             // bar[32]: own 128-byte line
-constexpr int kBarWords = 64;                              // words zeroed per launch
-
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -1627,7 +1654,9 @@ __device__ __forceinline__ void free_sweep(const StepArgs<Real>& a, const PRec<R
 template <typename Real, int MINB>
 __global__ void __launch_bounds__(kWinThreads, MINB) k_window(StepArgs<Real> a, int K, StepPartials part, size_t npart,
                                                            uint* bar) {
-    if (a.batch && !a.ccw[1]) return;   // the cluster batches (k_batch) step this window
+    // a batched window: the cluster batches (k_batch) step it, or the tiles
+    // (k_tile), unless one of those does not fit
+    if (a.batch && (!a.ccw[1] || (a.tw && !a.tw[kTwOver]))) return;
     uint nbar = 0;
     const uint nw = *a.wcount;
     const uint total = a.off[a.n];
@@ -2006,6 +2035,8 @@ __global__ void __maxnreg__(BatchRegs<Real>::value) k_batch(StepArgs<Real> a, in
     clear_partials(part, gridDim.x, clr1);
 }
 
+#include "dem_tile.cuh"
+
 // PP (particle-parallel, the paper's Figure 1(b)): each particle evaluates all
 // of its pairs itself -- its own row (it is lo) and its reverse row (it is hi)
 // -- and its walls, then integrates.  Each pair is evaluated by both of its
@@ -2259,55 +2290,57 @@ StepPartials free_partials(const dem_ctx* c, int slot) {
 // The outer build on stream st (plain launches: in a graph it is the body of
 // a conditional node): cells of the outer grid, their scan, the counting
 // scatter, the row lengths, their scan, the rows.
-template <typename Real> int outer_build(dem_ctx* c, const PRec<Real>* S, cudaStream_t st) {
+template <typename Real>
+int outer_build(dem_ctx* c, const PRec<Real>* S, cudaStream_t st, const uint* need = nullptr) {
     const long long n = c->n;
     const int B = 256;
     const GridC og = c->ogrid;
-    k_cell_hash<Real><<<grid_for(n, B), B, 0, st>>>(n, S, og, c->key, c->ccount, c->arrival);
+    k_cell_hash<Real><<<grid_for(n, B), B, 0, st>>>(n, S, og, c->key, c->ccount, c->arrival, need);
     DEM_LAUNCH_CHECK();
     int rc = exclusive_scan_u32(c->ccount, c->cstart, c->oncells, c->cstart + c->oncells, c->scan_tmp, st, false);
     if (rc) return rc;
     k_scatter<Real><<<grid_for(n, B), B, 0, st>>>(n, (const uint*)c->key, (const uint*)c->arrival,
                                                   (const uint*)c->cstart, c->ccount, S, (const Real*)c->rad, og,
-                                                  c->sid, c->skeyu, (R4<Real>*)c->sposu, c->tpos);
+                                                  c->sid, c->skeyu, (R4<Real>*)c->sposu, c->tpos, need);
     DEM_LAUNCH_CHECK();
     const Real oskin = (Real)c->oskin;
     k_outer_count<Real><<<grid_for(n, B), B, 0, st>>>(n, (const uint*)c->sid, (const R4<Real>*)c->sposu,
                                                       (const uint*)c->skeyu, (const uint*)c->cstart, og, oskin,
-                                                      c->ocnt);
+                                                      c->ocnt, need);
     DEM_LAUNCH_CHECK();
     if ((rc = exclusive_scan_u32(c->ocnt, c->coff, n, c->coff + n, c->scan_tmp, st, false))) return rc;
     k_outer_fill<Real><<<grid_for(n, B), B, 0, st>>>(n, (const uint*)c->sid, (const R4<Real>*)c->sposu,
                                                      (const uint*)c->skeyu, (const uint*)c->cstart, og, oskin,
                                                      (const uint*)c->coff, c->cln, c->ccap, S,
-                                                     planes<double>(c->xo, c->npad), c->oflag, c->words);
+                                                     planes<double>(c->xo, c->npad), c->oflag, c->words, need);
     DEM_LAUNCH_CHECK();
     return DEM_OK;
 }
 
-// In a capture: k_outer_check, then a conditional node whose body (captured
-// on the context's build stream) is the outer build; the capture goes on
-// after the node.
 template <typename Real>
 int launch_outer_check(dem_ctx* c, const PRec<Real>* S, cudaStream_t s, int cond, cudaGraphConditionalHandle h) {
     k_outer_check<Real><<<grid_for(c->n, 256), 256, 0, s>>>(
         c->n, S, (const Real*)c->rad, c->grid, c->cfg.world[0] * 0.5, c->cfg.world[1] * 0.5, 0.5 * c->cfg.skin,
-        c->ikey, planes<double>(c->xo, c->npad), c->odelta2, (const uint*)c->oflag, c->wcount, cond, h);
+        c->ikey, planes<double>(c->xo, c->npad), c->odelta2, c->oflag, c->wcount, cond, h);
     DEM_LAUNCH_CHECK();
     return DEM_OK;
 }
 
-template <typename Real> int outer_build_conditional(dem_ctx* c, const PRec<Real>* S) {
-    cudaStream_t s = c->stream;
+// A conditional (if) node after what stream s has captured so far: `body`
+// enqueues its graph on stream bs, and the capture goes on after the node.
+int conditional_handle(cudaStream_t s, cudaGraphConditionalHandle* h) {
+    cudaStreamCaptureStatus st;
+    cudaGraph_t cg = nullptr;
+    DEM_CUDA_TRY(cudaStreamGetCaptureInfo(s, &st, nullptr, &cg, nullptr, nullptr));
+    DEM_CUDA_TRY(cudaGraphConditionalHandleCreate(h, cg, 0, cudaGraphCondAssignDefault));
+    return DEM_OK;
+}
+
+template <typename F> int conditional_node(cudaStream_t s, cudaStream_t bs, cudaGraphConditionalHandle h, F body) {
     cudaStreamCaptureStatus st;
     cudaGraph_t cg = nullptr;
     const cudaGraphNode_t* deps = nullptr;
     size_t nd = 0;
-    DEM_CUDA_TRY(cudaStreamGetCaptureInfo(s, &st, nullptr, &cg, &deps, &nd));
-    cudaGraphConditionalHandle h;
-    DEM_CUDA_TRY(cudaGraphConditionalHandleCreate(&h, cg, 0, cudaGraphCondAssignDefault));
-    const int crc = launch_outer_check<Real>(c, S, s, 1, h);
-    if (crc) return crc;
     DEM_CUDA_TRY(cudaStreamGetCaptureInfo(s, &st, nullptr, &cg, &deps, &nd));
     cudaGraphNodeParams cp = {};
     cp.type = cudaGraphNodeTypeConditional;
@@ -2316,15 +2349,29 @@ template <typename Real> int outer_build_conditional(dem_ctx* c, const PRec<Real
     cp.conditional.size = 1;
     cudaGraphNode_t node;
     DEM_CUDA_TRY(cudaGraphAddNode(&node, cg, deps, nd, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    cudaGraph_t bg = cp.conditional.phGraph_out[0];
     DEM_CUDA_TRY(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
-    DEM_CUDA_TRY(cudaStreamBeginCaptureToGraph(c->cstream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    const int rc = outer_build<Real>(c, S, c->cstream);
+    DEM_CUDA_TRY(cudaStreamBeginCaptureToGraph(bs, bg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    const int rc = body();
     cudaGraph_t got = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(c->cstream, &got);
+    const cudaError_t e = cudaStreamEndCapture(bs, &got);
     if (rc) return rc;
-    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture (outer build)", __FILE__, __LINE__);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture (conditional body)", __FILE__, __LINE__);
     return DEM_OK;
+}
+
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusActive;
+}
+
+// In a capture: k_outer_check, then a conditional node whose body (captured
+// on the context's build stream) is the outer build.
+template <typename Real> int outer_build_conditional(dem_ctx* c, const PRec<Real>* S) {
+    cudaGraphConditionalHandle h;
+    int rc = conditional_handle(c->stream, &h);
+    if (rc || (rc = launch_outer_check<Real>(c, S, c->stream, 1, h))) return rc;
+    return conditional_node(c->stream, c->cstream, h, [&]() { return outer_build<Real>(c, S, c->cstream); });
 }
 
 template <typename Real> int launch_free(dem_ctx* c, int lst, int slot0, int nsteps, cudaStream_t s, int batch = 0);
@@ -2341,15 +2388,15 @@ template <typename Real> int launch_relist(dem_ctx* c, int src) {
     // predecessor before it touches memory, so only the launch latency overlaps
     const bool pdl = c->pdl && !c->profiling;
     // the outer list: rebuilt when needed (a graph's conditional node, switched
-    // by k_outer_check), always in an eager re-list
-    cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
-    DEM_CUDA_TRY(cudaStreamIsCapturing(s, &cst));
+    // by k_outer_check; an eager re-list's kernels read the check's word)
+    const bool graph = c->outer_cond && capturing(s);
     int rc;
-    if (cst == cudaStreamCaptureStatusActive && c->outer_cond) {
+    if (graph) {
         rc = outer_build_conditional<Real>(c, S);
     } else {
+        DEM_CUDA_TRY(cudaMemsetAsync(c->oflag + 1, 0, sizeof(uint), s));
         rc = launch_outer_check<Real>(c, S, s, 0, cudaGraphConditionalHandle{});
-        if (!rc) rc = outer_build<Real>(c, S, s);
+        if (!rc) rc = outer_build<Real>(c, S, s, c->oflag + 1);
     }
     if (rc) return rc;
     const Real skin = (Real)c->cfg.skin;
@@ -2388,13 +2435,17 @@ template <typename Real> int launch_relist(dem_ctx* c, int src) {
                            (const uint*)c->off[dst], c->cap, cc ? c->cc_parent : nullptr, (const uint*)c->bpos,
                            (const uint*)c->blist, c->cc_size, c->cc_pairs, (const uint*)c->cc_skip, c->cc_words));
     if (cc) {   // the window's components and batches (cluster-batched window path)
+        c->dense_cond = graph && c->window_follows;
+        c->dense_handle = cudaGraphConditionalHandle{};
+        if (c->dense_cond && (rc = conditional_handle(s, &c->dense_handle))) return rc;
         const uint* off = c->off[dst];
         const long long nbb = c->nbatch_max + 2;
         DEM_CUDA_TRY(launch_ex(k_cc_pass, BG, kCcThreads, s, pdl, n, c->cap, c->nbatch_max, nbb, c->batch_grid,
                                BatchCap<Real>::P, BatchCap<Real>::Q, off, (const uint*)c->bpos,
                                (const uint*)c->blist, (const uint*)c->cc_parent, (const uint*)c->cc_size,
                                (const uint*)c->cc_pairs, c->cc_base, c->cc_fill, c->cc_order, c->cc_bw, c->cc_batch,
-                               c->cc_words, c->cc_skip, c->lb + lb_cc(c->npad), c->words));
+                               c->cc_words, c->cc_skip, c->lb + lb_cc(c->npad), c->words,
+                               c->bar, c->dense_cond ? 1 : 0, c->dense_handle));
     }
     return DEM_OK;
 }
@@ -2430,6 +2481,7 @@ template <typename Real> StepArgs<Real> step_args(const dem_ctx* c, int lst, int
     a.split = c->win_split;
     a.batch = 0;
     a.ccw = c->cc_words;
+    a.tw = c->tw;
     a.words = c->words;
     a.dbgF = c->record ? c->dbgF : nullptr;
     a.dbgT = c->record ? c->dbgT : nullptr;
@@ -2472,9 +2524,11 @@ template <typename Real> int launch_free(dem_ctx* c, int lst, int slot0, int nst
 template <typename Real> auto window_fn(int minb) { return minb == 2 ? k_window<Real, 2> : k_window<Real, 1>; }
 
 // The window kernel: all K steps of the window in one cooperative launch.
-template <typename Real> int launch_window(dem_ctx* c, int lst, const WindowTape* tape, int batch = 0) {
+template <typename Real>
+int launch_window(dem_ctx* c, int lst, const WindowTape* tape, cudaStream_t s, int batch = 0) {
     const int K = c->cfg.relist_interval;
-    DEM_CUDA_TRY(cudaMemsetAsync(c->bar, 0, kBarWords * sizeof(uint), c->stream));   // counter, give-up word
+    if (!batch)   // counter, give-up word (cleared by the component pass in a batched window)
+        DEM_CUDA_TRY(cudaMemsetAsync(c->bar, 0, kBarWords * sizeof(uint), s));
     StepArgs<Real> a = step_args<Real>(c, lst, 0);
     a.batch = batch;
     a.dbgF = a.dbgT = nullptr;
@@ -2488,7 +2542,7 @@ template <typename Real> int launch_window(dem_ctx* c, int lst, const WindowTape
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(c->win_grid);
     cfg.blockDim = dim3(kWinThreads);
-    cfg.stream = c->stream;
+    cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
@@ -2523,14 +2577,74 @@ template <typename Real> int launch_window_pp(dem_ctx* c, int lst, int sb, int h
     return DEM_OK;
 }
 
-// The cluster-batched window: the grid-barrier window kernel (it steps the
-// window only when a component or batch is too large for a block), then the
-// free particles (forked stream) beside the batches, joined.
+// The tile arrays of context c as kernel arguments.
+template <typename Real> TileArgs<Real> tile_args(const dem_ctx* c) {
+    TileArgs<Real> T;
+    T.tw = c->tw; T.G = c->tile_grid; T.curve = c->tcurve; T.inv = c->tinv; T.flag = c->tflag; T.head = c->thead;
+    T.blob = c->tblob; T.tk = c->tk; T.twl = c->twl;
+    T.ts[0] = (PRec<Real>*)c->ts[0]; T.ts[1] = (PRec<Real>*)c->ts[1];
+    T.tq = c->tq;
+    T.th = Planes3<double>{c->thist[0], c->thist[1], c->thist[2]};
+    T.Q = c->tile_q;
+    T.BB = tile_blob(c->tile_q, TileCap<Real>::P);
+    return T;
+}
+
+// A window that the cluster batches do not step, on stream s (in a graph: the
+// body of a conditional node): the tiles' lists and the tiles' steps; the
+// grid-barrier window kernel only when a tile does not fit.
+template <typename Real> int launch_tiles(dem_ctx* c, int lst, const WindowTape* tape, cudaStream_t s) {
+    const int K = c->cfg.relist_interval;
+    if (c->tw) {
+        StepArgs<Real> a = step_args<Real>(c, lst, 0);
+        a.batch = 1;
+        a.dbgF = a.dbgT = nullptr;
+        a.dbgC = nullptr;
+        if (tape) {
+            a.tx = tape->tx; a.td = tape->td; a.twh = tape->twh; a.tF = tape->tF; a.tT = tape->tT; a.th = tape->th;
+            a.tc = tape->tc;
+            a.ta = (Real*)tape->ta;
+            a.tstep0 = tape->step0;
+        }
+        const TileArgs<Real> T = tile_args<Real>(c);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(c->tile_list_grid);
+        cfg.blockDim = dim3(TileCap<Real>::P);
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;   // every block resident: they wait for one another
+        at[0].val.cooperative = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        DEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_tile_lists<Real>, a, T, (const uint*)c->bflag, c->grid,
+                                        curve_grid(c->cfg.world, 2.0 * c->rmax), (uint)c->ntile_max, c->key,
+                                        c->arrival, c->cbin, c->cbin + c->ncbin, c->cbin + 2 * c->ncbin,
+                                        c->bar + kBarWords));
+        cfg.gridDim = dim3(c->tile_grid);
+        cfg.dynamicSmemBytes = TileCap<Real>::smem;
+        DEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, tape ? k_tile<Real, true> : k_tile<Real, false>, a, T, K,
+                                        partials(c, K - 1), (size_t)c->fpart, c->bar));
+    }
+    return launch_window<Real>(c, lst, tape, s, 1);
+}
+
+// The cluster-batched window: the batches beside the free particles (forked
+// stream), and beside them a conditional node that steps the window's bound
+// particles as tiles when a component or batch is too large for a block.
 template <typename Real> int launch_batched_window(dem_ctx* c, int lst, const WindowTape* tape) {
     const int K = c->cfg.relist_interval;
-    int rc = launch_window<Real>(c, lst, tape, 1);
-    if (rc) return rc;
+    int rc;
     if (!c->free_early) DEM_CUDA_TRY(cudaEventRecord(c->evfork, c->stream));
+    const bool graph = c->dense_cond && capturing(c->stream);
+    if (!graph && (rc = launch_tiles<Real>(c, lst, tape, c->stream))) return rc;
+    if (graph) {   // a branch of its own: the batches do not wait for it
+        DEM_CUDA_TRY(cudaEventRecord(c->evdense, c->stream));
+        DEM_CUDA_TRY(cudaStreamWaitEvent(c->stream3, c->evdense, 0));
+        rc = conditional_node(c->stream3, c->cstream, c->dense_handle,
+                              [&]() { return launch_tiles<Real>(c, lst, tape, c->cstream); });
+        if (rc) return rc;
+        DEM_CUDA_TRY(cudaEventRecord(c->evdjoin, c->stream3));
+    }
     StepArgs<Real> a = step_args<Real>(c, lst, 0);
     a.batch = 1;
     a.dbgF = a.dbgT = nullptr;
@@ -2564,6 +2678,7 @@ template <typename Real> int launch_batched_window(dem_ctx* c, int lst, const Wi
         DEM_CUDA_TRY(cudaEventRecord(c->evjoin, c->stream2));
     }
     DEM_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->evjoin, 0));
+    if (graph) DEM_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->evdjoin, 0));
     return DEM_OK;
 }
 
@@ -2594,7 +2709,8 @@ int window_kernel(dem_ctx* c, int lst, const WindowTape* tape) {
     if (use_batches(c))
         return c->prec == DEM_PREC_MIXED ? launch_batched_window<float>(c, lst, tape)
                                          : launch_batched_window<double>(c, lst, tape);
-    return c->prec == DEM_PREC_MIXED ? launch_window<float>(c, lst, tape) : launch_window<double>(c, lst, tape);
+    return c->prec == DEM_PREC_MIXED ? launch_window<float>(c, lst, tape, c->stream)
+                                      : launch_window<double>(c, lst, tape, c->stream);
 }
 
 int relist(dem_ctx* c, int src) {
@@ -2652,7 +2768,9 @@ int enqueue_window(dem_ctx* c, int src) {
     // a batched window: the free particles start inside the re-list
     c->free_early = c->free_fork > 0 && c->mode == DEM_FORCE_PCCP && !c->record && c->win_kernel && use_batches(c);
     c->observe_slot = K - 1;
+    c->window_follows = c->mode == DEM_FORCE_PCCP && !c->record && c->win_kernel && use_batches(c);
     int rc = relist(c, src);
+    c->window_follows = false;
     if (rc) { c->free_early = false; return rc; }
     if (wt) DEM_CUDA_TRY(cudaEventRecordWithFlags(c->wev[1], c->stream, cudaEventRecordExternal));
     c->hph = 0;
@@ -2705,13 +2823,35 @@ int enqueue_window(dem_ctx* c, int src) {
     return DEM_OK;
 }
 
-// Capture (once) and launch the window graph for the current buffers.
+// A layer that joins drops the window graphs (the particle count is part of
+// every captured launch), and the two graphs of the next particle count cost
+// ~0.9 ms to capture and instantiate; a window launched directly costs ~0.1 ms
+// of host time and runs through the outer build's launches (~20 us more).  So while the next layer
+// is fewer than kPourDirect windows away, a small system's windows are
+// launched directly (above 2^16 particles the extra passes over them cost
+// more).  2,000 spheres, a call of 200 steps that ends before the next layer:
+// 2.30 ms with the graphs, 1.70 direct.
+bool pour_due(const dem_ctx* c, long long s);
+constexpr int kPourDirect = 16;
+bool window_direct(const dem_ctx* c) {
+    if (!c->pouring || c->n >= c->ntot || c->n > 65536 || c->wtiming) return false;
+    return pour_due(c, c->step + (long long)kPourDirect * c->cfg.relist_interval - 1);
+}
+
+// Launch a whole window for the current buffers: its graph, captured once, or
+// (window_direct) its kernels.
 int launch_window_graph(dem_ctx* c) {
     NvtxRange r("dem window graph");
     const int src = c->cur, sb = c->sbuf, hp = c->hph;
     const int tm = c->wtiming ? 1 : 0;
     cudaGraphExec_t& ge = c->gexec[src][sb][hp][tm];
-    if (!ge) {
+    const bool direct = !ge && window_direct(c);
+    if (direct) {
+        const int rc = enqueue_window(c, src);
+        c->sbuf = sb;
+        c->hph = hp;
+        if (rc) return rc;
+    } else if (!ge) {
         cudaGraph_t g = nullptr;
         DEM_CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         c->wtiming_capture = tm != 0;
@@ -2727,7 +2867,7 @@ int launch_window_graph(dem_ctx* c) {
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate", __FILE__, __LINE__);
     }
-    DEM_CUDA_TRY(cudaGraphLaunch(ge, c->stream));
+    if (!direct) DEM_CUDA_TRY(cudaGraphLaunch(ge, c->stream));
     if (tm) c->wtiming_ran = true;
     const int K = c->cfg.relist_interval;
     c->hph = 0;
@@ -2747,6 +2887,14 @@ bool pour_due(const dem_ctx* c, long long s) {
     return time > (double)(float)c->n * c->pour_tnewpar / (double)(float)c->pour_nplayer;
 }
 
+// The particles' places changed altogether: the tiles' curve is computed at
+// the next window that uses it.
+int tiles_stale(dem_ctx* c) {
+    if (c->tw) DEM_CUDA_TRY(cudaMemsetAsync(c->tw + kTwValid, 0, sizeof(uint), c->stream));
+    if (c->cbin) DEM_CUDA_TRY(cudaMemsetAsync(c->cbin, 0, (size_t)c->ncbin * sizeof(uint), c->stream));
+    return DEM_OK;
+}
+
 // The next layer joins (dempacking.cu:459-461): nplayer more particles (the
 // rest at the end), and the step re-lists.
 int pour_insert(dem_ctx* c) {
@@ -2764,6 +2912,7 @@ int pour_insert(dem_ctx* c) {
     c->vol = 4.0 / 3.0 * M_PI * c->r3sum[nnew];
     c->in_window = 0;   // this step re-lists (m_hiall = 1)
     free_graphs(c);     // the particle count is part of every captured launch
+    if (const int rc = tiles_stale(c)) return rc;
     // the new particles have no outer rows yet
     DEM_CUDA_TRY(cudaMemsetAsync(c->oflag, 0x01, sizeof(uint), c->stream));
     return DEM_OK;
@@ -2784,6 +2933,78 @@ int host_perm(dem_ctx* c) {
     return DEM_OK;
 }
 }  // namespace dem
+
+// The tile path's arrays and launch shapes.  A context whose arrays do not
+// fit the device's memory goes without (c->tw stays null: such windows run
+// in the grid-barrier window kernel), as does one that re-lists every step
+// (the first and the last step of a window are then the same step, and a
+// pair across tiles would read a history that its owner writes).
+template <typename Real> int tiles_alloc(dem_ctx* c, cudaStream_t s) {
+    int nsm = 0, per[2] = {0, 0};
+    DEM_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+    const size_t smem = TileCap<Real>::smem;
+    void (*const fn[2])(StepArgs<Real>, TileArgs<Real>, int, StepPartials, size_t, uint*) = {k_tile<Real, false>,
+                                                                                             k_tile<Real, true>};
+    for (int k = 0; k < 2; k++) {
+        DEM_CUDA_TRY(cudaFuncSetAttribute(fn[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        DEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[k], fn[k], (int)TileCap<Real>::P, smem));
+    }
+    const int b = std::min(per[0], per[1]);
+    const long long np = c->npad;
+    if (b < 1 || c->cfg.relist_interval < 2) return DEM_OK;
+    const uint G = (uint)(nsm * b);
+    const long long nt = tile_max(c->ntot, G, TileCap<Real>::floor);
+    const size_t Q = c->ntot <= (long long)G * TileCap<Real>::P ? TileCap<Real>::Q1 : TileCap<Real>::Q2;
+    c->tile_q = (uint)Q;
+    // the histories between the steps go into the per-pair results of the
+    // grid-barrier kernels, which a tiled window does not use, when they fit
+    const bool alias = (size_t)nt * Q * sizeof(double) <= (size_t)c->cap * 4 * real_size(c->prec);
+    double* own = nullptr;
+    c->tile_grid = (unsigned)std::min<long long>(G, nt);
+    int lper = 0;
+    DEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lper, k_tile_lists<Real>, (int)TileCap<Real>::P, 0));
+    if (lper < 1) return DEM_OK;
+    c->tile_list_grid = (unsigned)std::min<long long>((long long)std::min(lper, 4) * nsm, nt);
+    c->ntile_max = nt;
+    struct Want { void** p; size_t bytes; };
+    const Want want[] = {{(void**)&c->tw, kTwWords * sizeof(uint)},
+                         {(void**)&c->tcurve, np * sizeof(uint)},
+                         {(void**)&c->tinv, np * sizeof(uint)},
+                         {(void**)&c->tflag, (size_t)nt * kFlagStride * sizeof(uint)},
+                         {(void**)&c->thead, 2 * nt * sizeof(uint4)},
+                         {(void**)&c->tblob, (size_t)nt * tile_blob((uint)Q, TileCap<Real>::P)},
+                         {(void**)&c->tk, nt * Q * sizeof(uint)},
+                         {(void**)&c->twl, (size_t)nt * TileCap<Real>::P * sizeof(unsigned short)},
+                         {(void**)&c->ts[0], np * sizeof(PRec<Real>)},
+                         {(void**)&c->ts[1], np * sizeof(PRec<Real>)},
+                         {(void**)&c->tq, np * sizeof(float4)},
+                         {(void**)&own, alias ? 0 : nt * Q * 3 * sizeof(double)}};
+    // one allocation (each cudaMalloc costs the set-up ~0.1 ms)
+    size_t total = 0;
+    for (const Want& w : want) total += (w.bytes + 255) / 256 * 256;
+    if (cudaMalloc((void**)&c->tmem, total) != cudaSuccess) {
+        cudaGetLastError();   // out of memory: no tiles
+        c->tmem = nullptr;
+        return DEM_OK;
+    }
+    size_t at = 0;
+    for (const Want& w : want) {
+        *w.p = c->tmem + at;
+        at += (w.bytes + 255) / 256 * 256;
+    }
+    if (alias) {
+        c->thist[0] = (double*)c->pti; c->thist[1] = (double*)c->rfj; c->thist[2] = (double*)c->rtj;
+    } else {
+        for (int k = 0; k < 3; k++) c->thist[k] = own + (size_t)k * nt * Q;
+    }
+    DEM_CUDA_TRY(cudaMemsetAsync(c->tw, 0, kTwWords * sizeof(uint), s));
+    c->tile_sms = nsm;
+    return DEM_OK;
+}
+
+int tiles_create(dem_ctx* c, cudaStream_t s) {
+    return c->prec == DEM_PREC_MIXED ? tiles_alloc<float>(c, s) : tiles_alloc<double>(c, s);
+}
 
 extern "C" {
 
@@ -2844,7 +3065,7 @@ int dem_create(const dem_config* cfg, dem_ctx** out) {
         (rc = dalloc(&c->rmax_bits, 3)) || (rc = dalloc(&c->wslot, np)) || (rc = dalloc(&c->wlist, np)) ||
         (rc = dalloc(&c->wcount, 1)) || (rc = dalloc(&c->arrival, np)) || (rc = dalloc(&c->scr, np * kScr)) ||
         (rc = dalloc(&c->bflag, np)) || (rc = dalloc(&c->bpos, np + 1)) || (rc = dalloc(&c->blist, np)) ||
-        (rc = dalloc(&c->flist, np)) || (rc = dalloc(&c->bar, kBarWords)) || (rc = dalloc(&c->tpos, np)))
+        (rc = dalloc(&c->flist, np)) || (rc = dalloc(&c->bar, 2 * kBarWords)) || (rc = dalloc(&c->tpos, np)))
         return bail(rc);
     // the outer candidate list (rows in both directions; its skin is set
     // with the grid, from r_max): four times the pair capacity
@@ -2936,9 +3157,10 @@ int dem_create(const dem_config* cfg, dem_ctx** out) {
             c->nbatch_max = (np + kBatchMin - 1) / kBatchMin + 1;
         }
     }
+    if (c->batching && (rc = tiles_create(c, s0))) return bail(rc);
     // partials per slot: the particle kernels' (at least as many as the
-    // window kernel has blocks), then the free kernel's
-    c->fpart = std::max<size_t>((size_t)c->nblk, c->win_grid);
+    // window kernels have blocks), then the free kernel's
+    c->fpart = std::max<size_t>((size_t)c->nblk, std::max(c->win_grid, c->tile_grid));
     c->npart = c->fpart + c->nblk;
     if ((rc = dalloc(&c->part_mz, (size_t)cfg->relist_interval * c->npart)) ||
         (rc = dalloc(&c->part_cnt, (size_t)cfg->relist_interval * c->npart)))
@@ -2962,7 +3184,7 @@ int dem_create(const dem_config* cfg, dem_ctx** out) {
     c->scan_words = 3 * scan_scratch_words(std::max<long long>(np + 1, 1));
     if ((rc = dalloc(&c->scan_tmp, c->scan_words))) return bail(rc);
     e = cudaMemsetAsync(c->words, 0, sizeof(EngineWords), s0);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->bar, 0, kBarWords * sizeof(uint), s0);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->bar, 0, 2 * kBarWords * sizeof(uint), s0);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->off[0], 0, (np + 1) * sizeof(uint), s0);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->off[1], 0, (np + 1) * sizeof(uint), s0);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->roff, 0, (np + 1) * sizeof(uint), s0);
@@ -2983,6 +3205,9 @@ int dem_create(const dem_config* cfg, dem_ctx** out) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->evfork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->evjoin, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->evdense, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->evdjoin, cudaEventDisableTiming);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate", __FILE__, __LINE__));
     e = cudaStreamSynchronize(s0);   // the initialisation above is done
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamSynchronize", __FILE__, __LINE__));
@@ -3004,7 +3229,7 @@ int dem_destroy(dem_ctx* c) {
                     c->part_cnt, c->rmax_bits, c->dbgF, c->dbgT, c->dbgC, c->wslot, c->wlist, c->wcount, c->wf, c->arrival,
                     c->scr, c->bflag, c->bpos, c->blist, c->flist, c->bar,
                     c->tpos, c->pour_rec, c->perm, c->cc_parent, c->cc_size, c->cc_base, c->cc_order,
-                    c->cc_batch, c->cc_loc, c->cc_words, c->cc_bw, c->cc_skip};
+                    c->cc_batch, c->cc_loc, c->cc_words, c->cc_bw, c->cc_skip, c->tmem, c->cbin};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c->host_pinned) cudaFreeHost(c->host_pinned);
@@ -3019,6 +3244,9 @@ int dem_destroy(dem_ctx* c) {
     for (cudaEvent_t e : c->wev) cudaEventDestroy(e);
     if (c->stream2) cudaStreamDestroy(c->stream2);
     if (c->cstream) cudaStreamDestroy(c->cstream);
+    if (c->stream3) cudaStreamDestroy(c->stream3);
+    if (c->evdense) cudaEventDestroy(c->evdense);
+    if (c->evdjoin) cudaEventDestroy(c->evdjoin);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
     return DEM_OK;
@@ -3098,6 +3326,24 @@ static int setup_grid(dem_ctx* c) {
     c->grid = g;
     c->ncells = nc;
     c->ogrid = og;
+    if (c->tw) {   // the tiles' curve bins: counts (zeroed), starts, block sums
+        const CurveGrid cg = curve_grid(c->cfg.world, 2.0 * c->rmax);
+        if (cg.nbins > c->ncbin) {
+            free_graphs(c);
+            if (c->cbin) {
+                DEM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+                cudaFree(c->cbin);
+                c->cbin = nullptr;
+                c->ncbin = 0;
+            }
+            const int rc = dalloc(&c->cbin, (size_t)2 * cg.nbins + (size_t)4 * c->tile_sms);
+            if (rc) return rc;
+            DEM_CUDA_TRY(cudaMemsetAsync(c->cbin, 0, (size_t)cg.nbins * sizeof(uint), c->stream));
+            c->ncbin = cg.nbins;
+        }
+        if (cg.cs != c->curve_cs) free_graphs(c);   // the cells' edge (r_max) is part of the captured launch
+        c->curve_cs = cg.cs;
+    }
     return DEM_OK;
 }
 
@@ -3107,6 +3353,7 @@ static int finish_upload(dem_ctx* c) {
     DEM_CUDA_TRY(cudaMemsetAsync(c->off[1], 0, (c->npad + 1) * sizeof(uint), c->stream));
     DEM_CUDA_TRY(cudaMemsetAsync(c->words, 0, sizeof(EngineWords), c->stream));
     if (c->cc_skip) DEM_CUDA_TRY(cudaMemsetAsync(c->cc_skip, 0, 2 * sizeof(uint), c->stream));
+    if (const int rc = tiles_stale(c)) return rc;
     // the outer list is rebuilt at the first re-list (new positions, radii)
     DEM_CUDA_TRY(cudaMemsetAsync(c->oflag, 0x01, sizeof(uint), c->stream));
     DEM_CUDA_TRY(cudaMemsetAsync(c->lb, 0, lb_words(c->npad) * sizeof(uint), c->stream));

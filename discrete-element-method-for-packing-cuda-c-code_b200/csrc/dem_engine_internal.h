@@ -39,46 +39,90 @@ template <> struct alignas(32) PRec<double> {
 };
 static_assert(sizeof(PRec<float>) == 64 && sizeof(PRec<double>) == 96, "record layout");
 
-// Record access by 16-byte vectors; COH: L2-coherent loads (.cg) for data that
-// other blocks of the same launch write.
 template <bool COH, typename T> __device__ __forceinline__ T ldv(const T* p) {
     if constexpr (COH) return __ldcg(p);
     else return *p;
 }
+
+// 32-byte global accesses (sm_100a): one request and one sector where two
+// 16-byte ones would each fetch the sector (L2-coherent loads bypass L1) and
+// each take a tag lookup per lane.  COH: L2-coherent (.cg), for data that
+// other blocks of the same launch write.
+struct Words4 { double a, b, c, d; };
+template <bool COH> __device__ __forceinline__ Words4 ld32(const void* p) {
+    Words4 v;
+    if constexpr (COH)
+        asm volatile("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p));
+    else
+        asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st32(void* p, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+__device__ __forceinline__ double f2d(float lo, float hi) { return __hiloint2double(__float_as_int(hi), __float_as_int(lo)); }
+__device__ __forceinline__ float d_lo(double v) { return __int_as_float(__double2loint(v)); }
+__device__ __forceinline__ float d_hi(double v) { return __int_as_float(__double2hiint(v)); }
+
+// Record access in global memory.
 template <bool COH>
 __device__ __forceinline__ void ld_rec(const PRec<float>* p, V3<double>& x, V3<double>& d, V3<float>& a, float& r) {
+    const Words4 u = ld32<COH>(p), w = ld32<COH>(reinterpret_cast<const char*>(p) + 32);
+    x = mk(u.a, u.b, u.c);
+    d = mk(u.d, w.a, w.b);
+    a = mk(d_lo(w.c), d_hi(w.c), d_lo(w.d));
+    r = d_hi(w.d);
+}
+template <bool COH>
+__device__ __forceinline__ void ld_rec(const PRec<double>* p, V3<double>& x, V3<double>& d, V3<double>& a,
+                                       double& r) {
+    const Words4 u = ld32<COH>(p), w = ld32<COH>(reinterpret_cast<const char*>(p) + 32);
+    const double2 v4 = ldv<COH>(reinterpret_cast<const double2*>(p) + 4);
+    x = mk(u.a, u.b, u.c);
+    d = mk(u.d, w.a, w.b);
+    a = mk(w.c, w.d, v4.x);
+    r = v4.y;
+}
+template <bool COH, typename Real> __device__ __forceinline__ V3<double> ld_pos(const PRec<Real>* p) {
+    const Words4 u = ld32<COH>(p);
+    return mk(u.a, u.b, u.c);
+}
+__device__ __forceinline__ void st_rec(PRec<float>* p, V3<double> x, V3<double> d, V3<float> a, float r) {
+    st32(p, x.x, x.y, x.z, d.x);
+    st32(reinterpret_cast<char*>(p) + 32, d.y, d.z, f2d(a.x, a.y), f2d(a.z, r));
+}
+__device__ __forceinline__ void st_rec(PRec<double>* p, V3<double> x, V3<double> d, V3<double> a, double r) {
+    st32(p, x.x, x.y, x.z, d.x);
+    st32(reinterpret_cast<char*>(p) + 32, d.y, d.z, a.x, a.y);
+    reinterpret_cast<double2*>(p)[4] = make_double2(a.z, r);
+}
+// The same layout in shared memory, by 16-byte words.
+__device__ __forceinline__ void lds_rec(const PRec<float>* p, V3<double>& x, V3<double>& d, V3<float>& a, float& r) {
     const double2* q = reinterpret_cast<const double2*>(p);
-    const double2 v0 = ldv<COH>(q), v1 = ldv<COH>(q + 1), v2 = ldv<COH>(q + 2);
-    const float4 v3 = ldv<COH>(reinterpret_cast<const float4*>(p) + 3);
+    const double2 v0 = q[0], v1 = q[1], v2 = q[2];
+    const float4 v3 = reinterpret_cast<const float4*>(p)[3];
     x = mk(v0.x, v0.y, v1.x);
     d = mk(v1.y, v2.x, v2.y);
     a = mk(v3.x, v3.y, v3.z);
     r = v3.w;
 }
-template <bool COH>
-__device__ __forceinline__ void ld_rec(const PRec<double>* p, V3<double>& x, V3<double>& d, V3<double>& a,
-                                       double& r) {
+__device__ __forceinline__ void lds_rec(const PRec<double>* p, V3<double>& x, V3<double>& d, V3<double>& a,
+                                        double& r) {
     const double2* q = reinterpret_cast<const double2*>(p);
-    const double2 v0 = ldv<COH>(q), v1 = ldv<COH>(q + 1), v2 = ldv<COH>(q + 2), v3 = ldv<COH>(q + 3),
-                  v4 = ldv<COH>(q + 4);
+    const double2 v0 = q[0], v1 = q[1], v2 = q[2], v3 = q[3], v4 = q[4];
     x = mk(v0.x, v0.y, v1.x);
     d = mk(v1.y, v2.x, v2.y);
     a = mk(v3.x, v3.y, v4.x);
     r = v4.y;
 }
-template <bool COH, typename Real> __device__ __forceinline__ V3<double> ld_pos(const PRec<Real>* p) {
-    const double2* q = reinterpret_cast<const double2*>(p);
-    const double2 v0 = ldv<COH>(q), v1 = ldv<COH>(q + 1);
-    return mk(v0.x, v0.y, v1.x);
-}
-__device__ __forceinline__ void st_rec(PRec<float>* p, V3<double> x, V3<double> d, V3<float> a, float r) {
+__device__ __forceinline__ void sts_rec(PRec<float>* p, V3<double> x, V3<double> d, V3<float> a, float r) {
     double2* q = reinterpret_cast<double2*>(p);
     q[0] = make_double2(x.x, x.y);
     q[1] = make_double2(x.z, d.x);
     q[2] = make_double2(d.y, d.z);
     reinterpret_cast<float4*>(p)[3] = make_float4(a.x, a.y, a.z, r);
 }
-__device__ __forceinline__ void st_rec(PRec<double>* p, V3<double> x, V3<double> d, V3<double> a, double r) {
+__device__ __forceinline__ void sts_rec(PRec<double>* p, V3<double> x, V3<double> d, V3<double> a, double r) {
     double2* q = reinterpret_cast<double2*>(p);
     q[0] = make_double2(x.x, x.y);
     q[1] = make_double2(x.z, d.x);
@@ -277,6 +321,29 @@ struct dem_ctx {
     long long nbatch_max = 0;
     unsigned batch_grid = 1;         // blocks of the batch kernel
     size_t batch_smem = 0;           // its dynamic shared memory
+    // tiles of a window whose components do not fit a block (dem_tile.cuh)
+    uint* tw = nullptr;              // the path's words (kTw...); null: no tiles
+    uint *tcurve = nullptr, *tinv = nullptr;   // np: particle by curve slot, slot by particle
+    uint *tflag = nullptr, *tk = nullptr;
+    uint4* thead = nullptr;
+    unsigned char* tblob = nullptr;
+    unsigned short* twl = nullptr;
+    void* ts[2] = {nullptr, nullptr};   // PRec<Real>[npad] by slot, step parity
+    float4* tq = nullptr;
+    double* thist[3] = {nullptr, nullptr, nullptr};   // planes (pti, rfj and rtj, or thist_own)
+    char* tmem = nullptr;            // the allocation that holds all of them
+    int tile_sms = 0;
+    double curve_cs = 0.0;           // edge of the curve's cells
+    uint tile_q = 0;
+    long long ntile_max = 0;
+    unsigned tile_grid = 1, tile_list_grid = 1;
+    uint* cbin = nullptr;            // the curve's bins: counts (ncbin), starts (ncbin), block sums
+    uint ncbin = 0;
+    bool window_follows = false;     // the re-list being enqueued is followed by a window (window_kernel)
+    bool dense_cond = false;         // capturing: the tiles are a conditional node, switched by the component pass
+    cudaGraphConditionalHandle dense_handle{};
+    cudaStream_t stream3 = 0;        // the tiles' branch of a window graph
+    cudaEvent_t evdense = nullptr, evdjoin = nullptr;
     uint* wslot = nullptr;   // per particle: wall-candidate slot of this window or kEmpty
     uint* wlist = nullptr;   // wall candidates (particle ids)
     uint* wcount = nullptr;  // number of wall candidates (device)
