@@ -1596,13 +1596,14 @@ __device__ __forceinline__ void free_item(const StepArgs<Real>& a, const PRec<Re
 
 // Free particles (flist[t], t < n - nB), slots slot0 .. slot0+nsteps-1.
 template <typename Real>
-__global__ void __launch_bounds__(256) k_free_run(StepArgs<Real> a, int slot0, int nsteps, int observe_slot,
-                                                  StepPartials part, size_t clr0, size_t clr1) {
+__global__ void __launch_bounds__(256) k_free_run(StepArgs<Real> a, const PRec<Real>* Sin, PRec<Real>* Sout, int slot0,
+                                                  int nsteps, int observe_slot, StepPartials part, size_t clr0,
+                                                  size_t clr1) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double mz_obs = 0.0;
     uint flags = 0;
     if (t < a.n - (long long)a.bpos[a.n])
-        free_item<Real>(a, a.S, a.S, a.flist[t], slot0, nsteps, observe_slot, a.dbgF != nullptr && nsteps == 1, mz_obs,
+        free_item<Real>(a, Sin, Sout, a.flist[t], slot0, nsteps, observe_slot, a.dbgF != nullptr && nsteps == 1, mz_obs,
                         flags);
     const int observe = observe_slot >= slot0 && observe_slot < slot0 + nsteps;
     block_observables(mz_obs, 0u, flags, observe, part, a.words);
@@ -2195,9 +2196,10 @@ template <typename Real>
 __global__ void __launch_bounds__(kWinThreads, 1) k_window_pp(StepArgs<Real> a, PRec<Real>* S0, PRec<Real>* S1,
                                                               Planes3<double> H0, Planes3<double> H1, int K,
                                                               StepPartials part, size_t npart, uint* bar) {
+    if (a.tw && !a.tw[kTwOver]) return;   // the tiles step this window
     uint nbar = 0;
     const uint total = a.off[a.n];
-    const long long nb = a.bpos[a.n], nf = a.n - nb;
+    const long long nb = a.bpos[a.n], nf = a.batch ? 0 : a.n - nb;   // batch: k_free_run steps the free particles
     const uint nbb = bound_blocks(nb, nb, nf, gridDim.x, a.split);
     const long long warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     PRec<Real>* Sf = (K & 1) ? S1 : S0;   // the free particles' final buffer
@@ -2583,7 +2585,11 @@ template <typename Real> int launch_free(dem_ctx* c, int lst, int slot0, int nst
     a.batch = batch;
     if (nsteps != 1) a.dbgF = a.dbgT = nullptr, a.dbgC = nullptr;
     const unsigned g = grid_for(c->n, 256);
-    k_free_run<Real><<<g, 256, 0, s>>>(a, slot0, nsteps, obs, free_partials(c, os), (size_t)g, (size_t)c->nblk);
+    // PP (whole windows only): from the window's first state buffer into its last
+    const PRec<Real>* Sin = c->mode == DEM_FORCE_PP ? (const PRec<Real>*)c->rec[c->sbuf] : a.S;
+    PRec<Real>* Sout = c->mode == DEM_FORCE_PP ? (PRec<Real>*)c->rec[(c->sbuf + nsteps) & 1] : a.S;
+    k_free_run<Real><<<g, 256, 0, s>>>(a, Sin, Sout, slot0, nsteps, obs, free_partials(c, os), (size_t)g,
+                                       (size_t)c->nblk);
     DEM_LAUNCH_CHECK();
     return DEM_OK;
 }
@@ -2624,12 +2630,17 @@ int launch_window(dem_ctx* c, int lst, const WindowTape* tape, cudaStream_t s, i
 }
 
 // PP window kernel: state buffer sb and history phase hp at the window start.
+template <typename Real> int launch_pp_tiles(dem_ctx* c, int lst, int sb, int hp);
 template <typename Real> int launch_window_pp(dem_ctx* c, int lst, int sb, int hp) {
     const int K = c->cfg.relist_interval;
-    DEM_CUDA_TRY(cudaMemsetAsync(c->bar, 0, kBarWords * sizeof(uint), c->stream));   // counter, give-up word
+    DEM_CUDA_TRY(cudaMemsetAsync(c->bar, 0, 2 * kBarWords * sizeof(uint), c->stream));   // counters, give-up words
     StepArgs<Real> a = step_args<Real>(c, lst, 0);
     a.dbgF = a.dbgT = nullptr;
     a.dbgC = nullptr;
+    if (c->tw) {
+        a.batch = 1;
+        if (const int rc = launch_pp_tiles<Real>(c, lst, sb, hp)) return rc;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(c->win_grid);
     cfg.blockDim = dim3(kWinThreads);
@@ -2641,8 +2652,8 @@ template <typename Real> int launch_window_pp(dem_ctx* c, int lst, int sb, int h
     cfg.numAttrs = 1;
     DEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_window_pp<Real>, a, (PRec<Real>*)c->rec[sb], (PRec<Real>*)c->rec[1 - sb],
                                     planes<double>(c->hist[lst][hp], c->cap),
-                                    planes<double>(c->hist[lst][1 - hp], c->cap), K, partials(c, K - 1), c->npart,
-                                    c->bar));
+                                    planes<double>(c->hist[lst][1 - hp], c->cap), K, partials(c, K - 1),
+                                    c->tw ? (size_t)c->fpart : c->npart, c->bar));
     return DEM_OK;
 }
 
@@ -2659,11 +2670,33 @@ template <typename Real> TileArgs<Real> tile_args(const dem_ctx* c) {
     return T;
 }
 
-// A window that the cluster batches do not step, on stream s (in a graph: the
-// body of a conditional node): the tiles' lists and the tiles' steps; the
-// grid-barrier window kernel only when a tile does not fit.
-template <typename Real> int launch_tiles(dem_ctx* c, int lst, const WindowTape* tape, cudaStream_t s) {
+// The tiles' lists and the tiles' steps (k_tile<Real, MODE>) of a window with
+// arguments a, on stream s.
+template <typename Real, int MODE>
+int launch_tile_kernels(dem_ctx* c, const StepArgs<Real>& a, const TileArgs<Real>& T, cudaStream_t s) {
     const int K = c->cfg.relist_interval;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(c->tile_list_grid);
+    cfg.blockDim = dim3(TileCap<Real>::P);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;   // every block resident: they wait for one another
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    DEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_tile_lists<Real, MODE == kTilePp>, a, T, (const uint*)c->bflag, c->grid,
+                                    curve_grid(c->cfg.world, 2.0 * c->rmax), (uint)c->ntile_max, c->key, c->arrival,
+                                    c->cbin, c->cbin + c->ncbin, c->cbin + 2 * c->ncbin, c->bar + kBarWords));
+    cfg.gridDim = dim3(c->tile_grid);
+    cfg.dynamicSmemBytes = TileCap<Real>::smem;
+    DEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_tile<Real, MODE>, a, T, K, partials(c, K - 1), (size_t)c->fpart, c->bar));
+    return DEM_OK;
+}
+
+// A window that the cluster batches do not step, on stream s (in a graph: the
+// body of a conditional node): the tiles, and the grid-barrier window kernel
+// only when a tile does not fit.
+template <typename Real> int launch_tiles(dem_ctx* c, int lst, const WindowTape* tape, cudaStream_t s) {
     if (c->tw) {
         StepArgs<Real> a = step_args<Real>(c, lst, 0);
         a.batch = 1;
@@ -2675,26 +2708,39 @@ template <typename Real> int launch_tiles(dem_ctx* c, int lst, const WindowTape*
             a.ta = (Real*)tape->ta;
             a.tstep0 = tape->step0;
         }
-        const TileArgs<Real> T = tile_args<Real>(c);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(c->tile_list_grid);
-        cfg.blockDim = dim3(TileCap<Real>::P);
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeCooperative;   // every block resident: they wait for one another
-        at[0].val.cooperative = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        DEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_tile_lists<Real>, a, T, (const uint*)c->bflag, c->grid,
-                                        curve_grid(c->cfg.world, 2.0 * c->rmax), (uint)c->ntile_max, c->key,
-                                        c->arrival, c->cbin, c->cbin + c->ncbin, c->cbin + 2 * c->ncbin,
-                                        c->bar + kBarWords));
-        cfg.gridDim = dim3(c->tile_grid);
-        cfg.dynamicSmemBytes = TileCap<Real>::smem;
-        DEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, tape ? k_tile<Real, true> : k_tile<Real, false>, a, T, K,
-                                        partials(c, K - 1), (size_t)c->fpart, c->bar));
+        TileArgs<Real> T = tile_args<Real>(c);
+        T.So = a.S;
+        T.Ho = a.H;
+        const int rc = tape ? launch_tile_kernels<Real, kTileTape>(c, a, T, s)
+                            : launch_tile_kernels<Real, kTilePccp>(c, a, T, s);
+        if (rc) return rc;
     }
     return launch_window<Real>(c, lst, tape, s, 1);
+}
+
+// A PP window's tiles beside its free particles (state buffer sb and history
+// phase hp at the window's start; both advance K steps); k_window_pp follows
+// and leaves at once unless a tile did not fit.
+template <typename Real> int launch_pp_tiles(dem_ctx* c, int lst, int sb, int hp) {
+    const int K = c->cfg.relist_interval;
+    StepArgs<Real> a = step_args<Real>(c, lst, 0);
+    a.batch = 1;
+    a.ccw = nullptr;
+    a.dbgF = a.dbgT = nullptr;
+    a.dbgC = nullptr;
+    a.S = (PRec<Real>*)c->rec[sb];
+    a.H = planes<double>(c->hist[lst][hp], c->cap);
+    TileArgs<Real> T = tile_args<Real>(c);
+    T.So = (PRec<Real>*)c->rec[(sb + K) & 1];
+    T.Ho = planes<double>(c->hist[lst][(hp + K) & 1], c->cap);
+    int rc;
+    DEM_CUDA_TRY(cudaEventRecord(c->evfork, c->stream));
+    DEM_CUDA_TRY(cudaStreamWaitEvent(c->stream2, c->evfork, 0));
+    if ((rc = launch_free<Real>(c, lst, 0, K, c->stream2, 1))) return rc;
+    DEM_CUDA_TRY(cudaEventRecord(c->evjoin, c->stream2));
+    if ((rc = launch_tile_kernels<Real, kTilePp>(c, a, T, c->stream))) return rc;
+    DEM_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->evjoin, 0));
+    return DEM_OK;
 }
 
 // The cluster-batched window: the batches beside the free particles (forked
@@ -3012,8 +3058,10 @@ template <typename Real> int tiles_alloc(dem_ctx* c, cudaStream_t s) {
     int nsm = 0, per[2] = {0, 0};
     DEM_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     const size_t smem = TileCap<Real>::smem;
-    void (*const fn[2])(StepArgs<Real>, TileArgs<Real>, int, StepPartials, size_t, uint*) = {k_tile<Real, false>,
-                                                                                             k_tile<Real, true>};
+    const bool pp = c->mode == DEM_FORCE_PP;
+    typedef void (*TileFn)(StepArgs<Real>, TileArgs<Real>, int, StepPartials, size_t, uint*);
+    const TileFn fn[2] = {pp ? (TileFn)k_tile<Real, kTilePp> : (TileFn)k_tile<Real, kTilePccp>,
+                          pp ? (TileFn)k_tile<Real, kTilePp> : (TileFn)k_tile<Real, kTileTape>};
     for (int k = 0; k < 2; k++) {
         DEM_CUDA_TRY(cudaFuncSetAttribute(fn[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         DEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[k], fn[k], (int)TileCap<Real>::P, smem));
@@ -3027,11 +3075,13 @@ template <typename Real> int tiles_alloc(dem_ctx* c, cudaStream_t s) {
     c->tile_q = (uint)Q;
     // the histories between the steps go into the per-pair results of the
     // grid-barrier kernels, which a tiled window does not use, when they fit
-    const bool alias = (size_t)nt * Q * sizeof(double) <= (size_t)c->cap * 4 * real_size(c->prec);
+    const bool alias = !pp && (size_t)nt * Q * sizeof(double) <= (size_t)c->cap * 4 * real_size(c->prec);
     double* own = nullptr;
     c->tile_grid = (unsigned)std::min<long long>(G, nt);
     int lper = 0;
-    DEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lper, k_tile_lists<Real>, (int)TileCap<Real>::P, 0));
+    DEM_CUDA_TRY(pp ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lper, k_tile_lists<Real, true>, (int)TileCap<Real>::P, 0)
+                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lper, k_tile_lists<Real, false>,
+                                                                    (int)TileCap<Real>::P, 0));
     if (lper < 1) return DEM_OK;
     c->tile_list_grid = (unsigned)std::min<long long>((long long)std::min(lper, 4) * nsm, nt);
     c->ntile_max = nt;
@@ -3226,7 +3276,8 @@ int dem_create(const dem_config* cfg, dem_ctx** out) {
             c->nbatch_max = (np + kBatchMin - 1) / kBatchMin + 1;
         }
     }
-    if (c->batching && (rc = tiles_create(c, s0))) return bail(rc);
+    // tiles: behind the cluster batches, and for every PP window
+    if ((c->batching || (c->mode == DEM_FORCE_PP && c->win_kernel)) && (rc = tiles_create(c, s0))) return bail(rc);
     // partials per slot: the particle kernels' (at least as many as the
     // window kernels have blocks), then the free kernel's
     c->fpart = std::max<size_t>((size_t)c->nblk, std::max(c->win_grid, c->tile_grid));
@@ -3405,7 +3456,7 @@ static int setup_grid(dem_ctx* c) {
                 c->cbin = nullptr;
                 c->ncbin = 0;
             }
-            const int rc = dalloc(&c->cbin, (size_t)2 * cg.nbins + (size_t)4 * c->tile_sms);
+            const int rc = dalloc(&c->cbin, (size_t)2 * cg.nbins + (size_t)8 * c->tile_sms);
             if (rc) return rc;
             DEM_CUDA_TRY(cudaMemsetAsync(c->cbin, 0, (size_t)cg.nbins * sizeof(uint), c->stream));
             c->ncbin = cg.nbins;

@@ -64,10 +64,10 @@ __host__ __device__ constexpr uint al16(uint b) { return (b + 15u) & ~15u; }
 // te, an entry per pair -- first the pairs inside the tile, lo | hi << 9 |
 // result << 18 (particles and result by their index in the tile), then those
 // across tiles, own particle | (1 << 9: it is hi) | result << 18 -- ; tx, the
-// partner's curve slot of each pair across tiles; tn, those tiles; tr, the reverse
+// partner's slot of each pair across tiles; tn, those tiles; tr, the reverse
 // rows as results; tp, per particle its row (first result | count << 16), its
 // reverse row (first in tr | count << 16), the result of its wall item
-// (kEmpty: none) and its id (kEmpty: not stepped).
+// (kEmpty: none) and its id.
 struct TileTables {
     uint ox, on, orr, op, bytes;
     __host__ __device__ TileTables(uint m, uint nin, uint tot, uint nrev, uint nnbr) {
@@ -83,21 +83,23 @@ __host__ __device__ constexpr uint tile_blob(uint q, uint p) { return q * 10u + 
 template <typename Real> struct TileArgs {
     uint* tw;
     uint G, Q, BB;           // resident blocks; the per-tile arrays' stride; bytes of a blob
-    uint* curve;             // particle id by curve slot
-    uint* inv;               // curve slot by particle id
+    uint* curve;             // every particle's id along the curve
+    uint* inv;               // a bound particle's slot: its place among the bound ones along the curve
     uint* flag;              // per tile (kFlagStride apart): steps finished in this window
-    uint4* head;             // per tile, two: pairs inside, all pairs, wall items, bound particles; reverse
-                             // entries, neighbour tiles
+    uint4* head;             // per tile, two: pairs inside, all pairs, wall items; reverse entries,
+                             // neighbour tiles
     unsigned char* blob;     // per tile: its tables
     uint* tk;                // per tile Q: a pair's slot in the list (top bit: the other tile owns its history)
     unsigned short* twl;     // per tile P: its wall items' particles
     PRec<Real>* ts[2];       // states by slot, step parity
     float4* tq;              // displacements since the list by slot
+    PRec<Real>* So;          // the states after the window
+    Planes3<double> Ho;      // the pair histories after the window
     Planes3<double> th;      // per tile Q: its pairs' histories between the first and the last step
 };
 
-// The window's tiles: particles per tile and shared memory of one stage
-// (states and tables).  f pairs per bound particle; a fraction c ~ 1.45 /
+// The window's tiles of its n bound particles: particles per tile and shared
+// memory of one stage (states and tables).  f pairs per particle; a fraction c ~ 1.45 /
 // P^(1/3) of a tile's pairs crosses its surface (a cube of P particles
 // loses 1.5 / P^(1/3)); 15 % of the pairs' bytes for uneven density, and
 // `shrink` sixteenths less after a window in which a tile did not fit.  One tile per
@@ -105,11 +107,11 @@ template <typename Real> struct TileArgs {
 // shared memory), else two stages per block (the next tile's loads run beside
 // the current one's steps), evened out over whole rounds of the G blocks.
 struct TilePlan { uint p, stage; };
-__host__ __device__ inline TilePlan tile_plan(long long n, long long pairs, long long nb, uint G, uint P, uint smem,
+__host__ __device__ inline TilePlan tile_plan(long long n, long long pairs, uint G, uint P, uint smem,
                                               uint rec, uint res, uint shrink) {
     TilePlan t{0u, 0u};
-    if (n <= 0 || nb <= 0 || shrink > 12u) return t;
-    const double f = 1.15 * (double)pairs / (double)nb;
+    if (n <= 0 || shrink > 12u) return t;
+    const double f = 1.15 * (double)pairs / (double)n;
     auto stage1 = [&](double p) {
         const double c = fmin(0.6, 1.45 / cbrt(p));
         return rec + 17.0 + 4.0 * f * (1.0 + c) + 8.0 * c * f + 2.0 * f;
@@ -206,17 +208,18 @@ __device__ __forceinline__ uint curve_bin(const V3<double>& p, const GridC& g, c
 
 // The window's tiles in one cooperative launch: their size, the step
 // counters; when the curve is missing or old, the particles' order along it (a
-// counting sort by bin, any order inside one); then each tile's lists, by one
+// counting sort by bin, any order inside one); the bound ones in that order,
+// numbered; then each tile's lists, by one
 // block: its pairs (the rows of its particles, and the reverse-row pairs
 // whose lower particle is in another tile), the tables above, the wall items,
 // and its particles' states in tile order.  One launch: as separate kernels
 // the window graph took 24 more nodes, 90 us longer to instantiate.
-template <typename Real>
+template <typename Real, bool PP>
 __global__ void __launch_bounds__(TileCap<Real>::P)
     k_tile_lists(StepArgs<Real> a, TileArgs<Real> T, const uint* __restrict__ bflag, GridC g, CurveGrid cg, uint ntmax,
-                 uint* __restrict__ key, uint* __restrict__ arrival, uint* __restrict__ count, uint* __restrict__ start,
+                 uint* key, uint* __restrict__ arrival, uint* __restrict__ count, uint* __restrict__ start,
                  uint* __restrict__ bsum, uint* bar) {
-    if (!a.ccw[1]) return;   // the cluster batches step this window
+    if (a.ccw && !a.ccw[1]) return;   // the cluster batches step this window
     const uint Q = T.Q;
     constexpr uint PC = TileCap<Real>::P;
     constexpr uint kTileThreads = PC;
@@ -226,32 +229,33 @@ __global__ void __launch_bounds__(TileCap<Real>::P)
     __shared__ uint s_tmp[34], s_hash[kTileHash], s_nbr[kTileNbr], s_nn;
     const uint p = threadIdx.x, nthr = gridDim.x * kTileThreads, gid = blockIdx.x * kTileThreads + p;
     const long long n = a.n;
+    const uint nbound = a.bpos[n];
     uint nbar = 0;
     for (uint t = gid; t < ntmax; t += nthr) T.flag[(size_t)t * kFlagStride] = 0u;
     if (gid == 0) {
-        const long long pairs = a.off[n], nb = a.bpos[n];
+        const long long pairs = a.off[n];
         uint shrink = T.tw[kTwShrink];
         if (T.tw[kTwOver] == 2u) T.tw[kTwShrink] = ++shrink;   // the last window's tiles did not fit
         TilePlan pl{0u, 0u};
         if (pairs <= a.cap)
-            pl = tile_plan(n, pairs, nb, T.G, PC, TileCap<Real>::smem, (uint)sizeof(TileRec<Real>), RB, shrink);
-        const uint nt = pl.p ? (uint)((n + pl.p - 1) / pl.p) : 0u;
-        const bool fits = pl.p && nt <= ntmax;
+            pl = tile_plan((long long)nbound, pairs, T.G, PC, TileCap<Real>::smem, (uint)sizeof(TileRec<Real>), RB, shrink);
+        const uint nt = pl.p ? (nbound + pl.p - 1) / pl.p : 0u;
+        const bool fits = nbound == 0u || (pl.p && nt <= ntmax);
         T.tw[kTwP] = pl.p;
         T.tw[kTwTiles] = nt;
         T.tw[kTwStage] = pl.stage;
         T.tw[kTwOver] = fits ? 0u : 1u;
         const uint age = T.tw[kTwAge];
         const bool need = !T.tw[kTwValid] || age >= kCurveEvery;
-        T.tw[kTwNeed] = need && fits ? 1u : 0u;
-        if (fits) {
+        T.tw[kTwNeed] = need && fits && nt ? 1u : 0u;
+        if (fits && nt) {
             T.tw[kTwAge] = need ? 1u : age + 1u;
             T.tw[kTwValid] = 1u;
         }
     }
     grid_barrier(bar, nbar++, gridDim.x, a.words);
     const uint PT = __ldcg(T.tw + kTwP), nt = __ldcg(T.tw + kTwTiles), stage = __ldcg(T.tw + kTwStage);
-    if (PT == 0u || nt > ntmax) return;
+    if (PT == 0u || nt == 0u || nt > ntmax) return;
     if (__ldcg(T.tw + kTwNeed)) {
         for (long long i = gid; i < n; i += nthr) {
             const uint c = curve_bin(ld_pos<false>(a.S + i), g, cg);
@@ -287,26 +291,51 @@ __global__ void __launch_bounds__(TileCap<Real>::P)
             const uint t = __ldcg(start + key[i]) + arrival[i];
             if ((long long)t >= n) continue;   // cannot happen (counts left over from a wait that gave up)
             T.curve[t] = (uint)i;
-            T.inv[i] = t;
         }
         grid_barrier(bar, nbar++, gridDim.x, a.words);
-        if (ld_acquire(bar + kBarGiveUp)) {   // no order along the curve: the grid-barrier kernel has the window
-            if (p == 0) { T.tw[kTwOver] = 1u; T.tw[kTwValid] = 0u; }
-            return;
+    }
+    // the bound particles along the curve: their ids (bl) and their slots
+    uint* bl = key;
+    {
+        const uint per = (uint)((n + gridDim.x - 1) / gridDim.x);
+        const uint b0 = (uint)min(n, (long long)blockIdx.x * per), b1 = (uint)min(n, (long long)b0 + per);
+        uint v = 0;
+        for (uint k = b0 + p; k < b1; k += kTileThreads) v += bflag[__ldcg(T.curve + k)];
+        s_own[p] = v;
+        const uint mine = block_exscan(s_own, s_ob, kTileThreads, s_tmp);
+        uint* bs = bsum + gridDim.x;   // the curve's sums may still be read
+        if (p == 0) bs[blockIdx.x] = mine;
+        grid_barrier(bar, nbar++, gridDim.x, a.words);
+        v = 0;
+        for (uint k = p; k < blockIdx.x; k += kTileThreads) v += __ldcg(bs + k);
+        s_own[p] = v;
+        uint run = block_exscan(s_own, s_ob, kTileThreads, s_tmp);
+        for (uint k0 = b0; k0 < b1; k0 += kTileThreads) {
+            const uint k = k0 + p, i = k < b1 ? __ldcg(T.curve + k) : 0u;
+            const uint on = k < b1 ? bflag[i] : 0u;
+            s_own[p] = on;
+            const uint sum = block_exscan(s_own, s_ob, kTileThreads, s_tmp);
+            if (on && run + s_ob[p] < nbound) {
+                bl[run + s_ob[p]] = i;
+                T.inv[i] = run + s_ob[p];
+            }
+            run += sum;
         }
+        grid_barrier(bar, nbar++, gridDim.x, a.words);
+    }
+    if (ld_acquire(bar + kBarGiveUp)) {   // the orders may be incomplete: the grid-barrier kernel has the window
+        if (p == 0) { T.tw[kTwOver] = 1u; T.tw[kTwValid] = 0u; }
+        return;
     }
     for (uint t = blockIdx.x; t < nt; t += gridDim.x) {
         const uint first = t * PT, slot = first + p;
-        const uint m = min(PT, (uint)n - first);
+        const uint m = min(PT, nbound - first);
         uint id = kEmpty, o0 = 0, no = 0, r0 = 0, nr = 0, nc = 0, ni = 0, ws = kEmpty;
         if (p < m) {
-            const uint i = __ldcg(T.curve + slot);
-            if (bflag[i]) {
-                id = i;
-                o0 = a.off[i]; no = a.off[i + 1] - o0;
-                r0 = a.roff[i]; nr = a.roff[i + 1] - r0;
-                ws = a.wslot[i];
-            }
+            id = __ldcg(bl + slot);
+            o0 = a.off[id]; no = a.off[id + 1] - o0;
+            r0 = a.roff[id]; nr = a.roff[id + 1] - r0;
+            if (!PP) ws = a.wslot[id];   // PP: a particle steps its walls itself
         }
         for (uint e = 0; e < no; e++) ni += __ldcg(T.inv + a.ln[o0 + e]) - first < m ? 1u : 0u;   // unsigned: inside the tile
         for (uint u = 0; u < nr; u++) nc += __ldcg(T.inv + a.lp[a.rk[r0 + u]]) - first < m ? 0u : 1u;
@@ -318,7 +347,7 @@ __global__ void __launch_bounds__(TileCap<Real>::P)
         s_hb[p] = no - ni + nc;
         s_rb[p] = nr;
         s_wb[p] = ws != kEmpty ? 1u : 0u;
-        const uint nbnd = (uint)__syncthreads_count(id != kEmpty);
+        __syncthreads();
         const uint town = block_exscan(s_own, s_ob, kTileThreads, s_tmp);
         const uint tcross = block_exscan(s_cb, s_cb, kTileThreads, s_tmp);
         const uint tin = block_exscan(s_ib, s_ib, kTileThreads, s_tmp);
@@ -398,17 +427,15 @@ __global__ void __launch_bounds__(TileCap<Real>::P)
         if (ws != kEmpty) T.twl[(size_t)t * PC + s_wb[p]] = (unsigned short)p;
         if (p < m) {
             tp[p] = make_uint4(s_ob[p] | (no << 16), s_rb[p] | (nr << 16), ws != kEmpty ? tot + s_wb[p] : kEmpty, id);
-            if (id != kEmpty) {
-                V3<double> x, d;
-                V3<Real> av;
-                Real r;
-                ld_rec<false>(a.S + id, x, d, av, r);
-                st_rec(T.ts[0] + slot, x, d, av, r);
-                T.tq[slot] = a.Q[id];
-            }
+            V3<double> x, d;
+            V3<Real> av;
+            Real r;
+            ld_rec<false>(a.S + id, x, d, av, r);
+            st_rec(T.ts[0] + slot, x, d, av, r);
+            T.tq[slot] = a.Q[id];
         }
         if (p == 0) {
-            T.head[2 * (size_t)t] = make_uint4(tin, tot, twall, nbnd);
+            T.head[2 * (size_t)t] = make_uint4(tin, tot, twall, 0u);
             T.head[2 * (size_t)t + 1] = make_uint4(trev, nnbr, 0u, 0u);
         }
         __syncthreads();   // the shared arrays are the next tile's
@@ -498,10 +525,18 @@ __device__ __forceinline__ void tile_stage(const TileArgs<Real>& T, uint t, uint
     for (uint c = threadIdx.x; c < L.bytes / 16u; c += NT) cp16(d2 + 16u * c, B + 16u * c);
 }
 
-template <typename Real, bool TAPE>
+// MODE: the PCCP window, the same writing the adjoint's tape, or the PP window
+// (k_window_pp, one thread through all of a sphere's pairs twice over, took 771
+// us per 20-step window of a 60,001-sphere bed, this 226 and 50 for the lists)
+// (a pair's force subtracted on hi; each particle's walls evaluated after its
+// pairs and gravity, added to its force wall by wall, as pp_item and
+// particle_finish do).
+enum : int { kTilePccp = 0, kTileTape = 1, kTilePp = 2 };
+template <typename Real, int MODE>
 __global__ void __maxnreg__(TileCap<Real>::regs)
     k_tile(StepArgs<Real> a, TileArgs<Real> T, int K, StepPartials part, size_t clr1, uint* bar) {
-    if (!a.ccw[1] || T.tw[kTwOver]) return;
+    constexpr bool TAPE = MODE == kTileTape, PP = MODE == kTilePp;
+    if ((a.ccw && !a.ccw[1]) || T.tw[kTwOver]) return;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(8) unsigned long long s_ready;
     const uint Q = T.Q;
@@ -511,14 +546,10 @@ __global__ void __maxnreg__(TileCap<Real>::regs)
     typedef typename Two<Real>::T R2;
     const uint PT = T.tw[kTwP], nt = T.tw[kTwTiles], stage = T.tw[kTwStage], tid = threadIdx.x;
     R2* res = reinterpret_cast<R2*>(smem + (nt <= gridDim.x ? 1u : 2u) * stage);
-    // this block's tiles with bound particles (another has no pairs, so no
-    // tile waits for it): a block with one keeps its states in shared memory
-    uint mine = 0, t = 0;
-    for (uint x = blockIdx.x; x < nt; x += gridDim.x)
-        if (T.head[2 * (size_t)x].w) {
-            if (mine == 0) t = x;
-            mine++;
-        }
+    // this block's tiles: a block with one keeps its states in shared memory
+    const uint nbound = a.bpos[a.n];
+    uint t = blockIdx.x;
+    const uint mine = t < nt ? (nt - t + gridDim.x - 1) / gridDim.x : 0u;
     double mz = 0.0;
     uint cnt = 0, flags = 0;
     if (mine) {
@@ -530,7 +561,7 @@ __global__ void __maxnreg__(TileCap<Real>::regs)
         uint tp0 = t;   // the tile stepped last, and the steps it has finished
         int sdone = 0;
         if (tid == 0) ready_init(&s_ready);
-        tile_stage<Real>(T, t, hd, hx, t * PT, min(PT, (uint)a.n - t * PT), T.ts[0], smem);
+        tile_stage<Real>(T, t, hd, hx, t * PT, min(PT, nbound - t * PT), T.ts[0], smem);
         for (int s = 0; s < K;) {
             const bool last = s == K - 1;
             pc.first = s == 0 ? 1 : 0;
@@ -538,7 +569,7 @@ __global__ void __maxnreg__(TileCap<Real>::regs)
             const PRec<Real>* cur = (s & 1) ? T.ts[1] : T.ts[0];
             PRec<Real>* nxt = (s & 1) ? T.ts[0] : T.ts[1];
             const uint first = t * PT;
-            const uint m = min(PT, (uint)a.n - first);
+            const uint m = min(PT, nbound - first);
             const uint nin = hd.x, tot = hd.y, nitem = hd.y + hd.z;
             unsigned char* S = smem + sb * stage;
             const TileTables L(m, nin, tot, hx.x, hx.y);
@@ -557,16 +588,14 @@ __global__ void __maxnreg__(TileCap<Real>::regs)
             uint4 hn = hd;
             uint4 hxn = hx;
             if (mine > 1) {
-                do {
-                    tn += gridDim.x;
-                    if (tn >= nt) tn = blockIdx.x;
-                    hn = T.head[2 * (size_t)tn];
-                } while (!hn.w);
+                tn += gridDim.x;
+                if (tn >= nt) tn = blockIdx.x;
+                hn = T.head[2 * (size_t)tn];
                 sn = tn > t ? s : s + 1;
                 hxn = T.head[2 * (size_t)tn + 1];
                 if (sn < K) {
                     sb ^= 1u;
-                    tile_stage<Real>(T, tn, hn, hxn, tn * PT, min(PT, (uint)a.n - tn * PT),
+                    tile_stage<Real>(T, tn, hn, hxn, tn * PT, min(PT, nbound - tn * PT),
                                      (sn & 1) ? T.ts[1] : T.ts[0], smem + sb * stage);
                 }
             }
@@ -635,7 +664,7 @@ __global__ void __maxnreg__(TileCap<Real>::regs)
                         Tj = Ti;
                     }
                     if (last) {
-                        if (own) { a.H.x[k] = h.x; a.H.y[k] = h.y; a.H.z[k] = h.z; }
+                        if (own) { T.Ho.x[k] = h.x; T.Ho.y[k] = h.y; T.Ho.z[k] = h.z; }
                     } else {
                         hx0[u] = h.x; hy0[u] = h.y; hz0[u] = h.z;
                     }
@@ -707,7 +736,20 @@ __global__ void __maxnreg__(TileCap<Real>::regs)
                     if (count) ci += v4.y != (Real)0 ? 1u : 0u;
                 }
                 F.z += -sphere_mass(a.density, r);
-                if (tp.z != kEmpty) {
+                const Real mass = sphere_mass(a.density, r);
+                uint wflag = __float_as_uint(q.w);
+                if (PP) {
+                    const double rd = (double)r;
+                    const bool touch = (x.z < rd) || (x.x + pc.hx < rd) || (pc.hx - x.x < rd) || (x.y + pc.hy < rd) ||
+                                       (pc.hy - x.y < rd);
+                    if (touch || wflag) {
+                        V3<double> hw = wflag ? ld3p<true>(a.W, i) : zero3<double>();
+                        const int hit = wall_contacts<Real>(pc.hx, pc.hy, x, cvt<Real>(d), av, r, mass, hw, a.inv_dt, a.pw,
+                                                            F, M, (Real*)nullptr);
+                        a.W.x[i] = hw.x; a.W.y[i] = hw.y; a.W.z[i] = hw.z;
+                        wflag = hit ? 1u : 0u;
+                    }
+                } else if (tp.z != kEmpty) {
                     const R2* o = res + 5 * tp.z;
                     const R2 v0 = o[0], v1 = o[1], v2 = o[2];
                     F.x += v0.x; F.y += v0.y; F.z += v1.x;
@@ -720,15 +762,13 @@ __global__ void __maxnreg__(TileCap<Real>::regs)
                     g[3 * i] = M.x; g[3 * i + 1] = M.y; g[3 * i + 2] = M.z;
                     a.tc[a.tnp * ts + i] = ci;
                 }
-                const Real mass = sphere_mass(a.density, r);
                 const Real I = (Real)0.4 * mass * (r * r);
                 if (pc.first) { q.x = 0.f; q.y = 0.f; q.z = 0.f; }
-                const float wflag = q.w;
                 double mzi;
                 integrate<Real>(F, M, mass, I, pc.dt, a.dtr, pc.half_skin2, x, d, av, q, flags, mzi);
-                q.w = wflag;
+                q.w = __uint_as_float(wflag);
                 if (last) {
-                    st_rec(a.S + i, x, d, av, r);
+                    st_rec(T.So + i, x, d, av, r);
                     a.Q[i] = q;
                     mz = fmax(mz, mzi);
                     cnt += ci;

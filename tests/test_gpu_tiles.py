@@ -1,6 +1,7 @@
 """Windows whose components do not fit a block, stepped as tiles
 (csrc/dem_tile.cuh), against the grid-barrier window kernel
-(DEM_B200_BATCH=0): the same states, pair lists with their histories and
+(DEM_B200_BATCH=0), in PP mode against the per-step kernels
+(DEM_B200_WINDOW=0): the same states, pair lists with their histories and
 observables, bit for bit -- one tile, tiles that stay in shared memory, blocks
 that stream several tiles or have one while others have two, long rows (a
 close-packed crystal), a density so uneven that the first window's tiles do
@@ -37,8 +38,8 @@ def crystal(dem, wl, nx, ny, nz, loose=0):
                        60, 20, 0.05, dem.PREC_FP64, pp, pw)
 
 
-def run(dem, w, prec, K, steps, motion, adjoint=0):
-    e = dem.Engine(**{**w.engine_kwargs(), "precision": prec, "relist_interval": K})
+def run(dem, w, prec, K, steps, motion, adjoint=0, mode=0):
+    e = dem.Engine(**{**w.engine_kwargs(), "precision": prec, "relist_interval": K, "force_mode": mode})
     e.set_material(w.pp, w.pw)
     e.upload(w.pos, w.rad, *motion)
     if adjoint:
@@ -54,14 +55,15 @@ def run(dem, w, prec, K, steps, motion, adjoint=0):
     return out, [s[k] for k in ("pairs", "contacts", "maxhz", "status")], work
 
 
-def check(dem, w, prec, monkeypatch, K=20, steps=60, adjoint=0):
+def check(dem, w, prec, monkeypatch, K=20, steps=60, adjoint=0, mode=0):
     rng = np.random.default_rng(9)
     motion = [1e-5 * (rng.random(3 * w.n) - 0.5) for _ in range(2)]
-    a, sa, work = run(dem, w, prec, K, steps, motion, adjoint)
-    monkeypatch.setenv("DEM_B200_BATCH", "0")
-    b, sb, _ = run(dem, w, prec, K, steps, motion, adjoint)
-    monkeypatch.delenv("DEM_B200_BATCH")
-    assert work["batched"] == 0 and sa[3] == 0
+    a, sa, work = run(dem, w, prec, K, steps, motion, adjoint, mode)
+    switch = "DEM_B200_WINDOW" if mode else "DEM_B200_BATCH"
+    monkeypatch.setenv(switch, "0")
+    b, sb, _ = run(dem, w, prec, K, steps, motion, adjoint, mode)
+    monkeypatch.delenv(switch)
+    assert work["batched"] == (-1 if mode else 0) and sa[3] == 0
     assert sa == sb
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x, y)
@@ -89,3 +91,37 @@ def test_crystal(dem, wl, cuda, monkeypatch, prec, size, loose):
 @pytest.mark.parametrize("prec", [0, 1])
 def test_adjoint_tape(dem, cuda, monkeypatch, prec):
     check(dem, dense_lattice(dem, 14, 14, 12), prec, monkeypatch, steps=40, adjoint=20)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("K", [2, 3, 20])
+def test_pp(dem, cuda, monkeypatch, prec, K):
+    """The particle-parallel mode, an odd and an even number of steps per
+    window (the state and history buffers alternate)."""
+    check(dem, dense_lattice(dem, 14, 14, 12), prec, monkeypatch, K=K, steps=5 * K, mode=1)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_pp_large_and_uneven(dem, wl, cuda, monkeypatch, prec):
+    check(dem, dense_lattice(dem, 44, 44, 40), prec, monkeypatch, steps=40, mode=1)
+    check(dem, crystal(dem, wl, 24, 24, 20, loose=20000), prec, monkeypatch, steps=60, mode=1)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_mostly_free(dem, wl, cuda, monkeypatch, prec, mode):
+    """A small crystal under a dilute cloud: few bound particles among many,
+    and none at all."""
+    w = crystal(dem, wl, 14, 14, 12)
+    rng = np.random.default_rng(5)
+    k = np.arange(30000)
+    cloud = np.stack([(k % 30) * 2.0 - 29, (k // 30 % 30) * 2.0 - 29, 30 + (k // 900) * 2.0], 1)
+    cloud += rng.uniform(-0.3, 0.3, cloud.shape)
+    w.pos = np.concatenate([w.pos, cloud.reshape(-1)])
+    w.rad = np.concatenate([w.rad, np.full(k.size, 0.5)])
+    w.n = w.rad.size
+    w.world = (64.0, 64.0, 120.0)
+    check(dem, w, prec, monkeypatch, steps=60, mode=mode)
+    if mode:
+        w.pos, w.rad, w.n = w.pos[-3 * k.size:].copy(), w.rad[-k.size:].copy(), k.size
+        check(dem, w, prec, monkeypatch, steps=40, mode=mode)
