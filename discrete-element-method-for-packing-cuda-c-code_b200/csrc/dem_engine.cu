@@ -3349,7 +3349,7 @@ int dem_destroy(dem_ctx* c) {
                     c->part_cnt, c->rmax_bits, c->dbgF, c->dbgT, c->dbgC, c->wslot, c->wlist, c->wcount, c->wf, c->arrival,
                     c->scr, c->bflag, c->bpos, c->blist, c->flist, c->bar,
                     c->tpos, c->pour_rec, c->perm, c->cc_parent, c->cc_size, c->cc_base, c->cc_order,
-                    c->cc_batch, c->cc_loc, c->cc_words, c->cc_bw, c->cc_skip, c->tmem, c->cbin};
+                    c->cc_batch, c->cc_loc, c->cc_words, c->cc_bw, c->cc_skip, c->tmem, c->cbin, c->sort_tmp};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c->host_pinned) cudaFreeHost(c->host_pinned);
@@ -3534,18 +3534,16 @@ static int device_cell_order(dem_ctx* c, const double* pos, long long n, bool* o
     const long long np = c->npad;
     uint2* kv = reinterpret_cast<uint2*>(c->scr);   // 2 np words
     uint2* kv2 = kv + np;                            // 2 np words
-    uint* scratch = c->scr + 4 * np;                 // (kScr - 4) np words
-    // the sort's histograms fit the rest of the scratch from 65 particles on;
-    // fewer keep the caller's order
-    if (radix_scratch_words((uint)n) > (size_t)(kScr - 4) * (size_t)np) return DEM_OK;
+    if (n < 65) return DEM_OK;   // fewer keep the caller's order
     int rc;
     if (!c->perm && (rc = dalloc(&c->perm, np))) return rc;
+    if (!c->sort_tmp && (rc = dalloc(&c->sort_tmp, radix_scratch_words((uint)c->ntot)))) return rc;
     k_cell_keys<<<grid_for(n, 256), 256, 0, c->stream>>>(n, pos, cs, 0.5 * c->cfg.world[0], 0.5 * c->cfg.world[1],
                                                          gx, gy, gz, kv);
     DEM_LAUNCH_CHECK();
     uint bits = 1;
     while (bits < 32 && (1ull << bits) < (unsigned long long)nc) bits++;
-    if ((rc = radix_sort_pairs(kv, kv2, (uint)n, bits, scratch, c->stream))) return rc;
+    if ((rc = radix_sort_pairs(kv, kv2, (uint)n, bits, c->sort_tmp, c->stream))) return rc;
     k_perm_of<<<grid_for(n, 256), 256, 0, c->stream>>>(n, kv, c->perm);
     DEM_LAUNCH_CHECK();
     c->hperm_stale = true;

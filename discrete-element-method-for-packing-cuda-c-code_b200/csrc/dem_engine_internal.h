@@ -226,6 +226,7 @@ struct dem_ctx {
     bool reorder = true;                   // host uploads sort by cell (DEM_B200_REORDER=0: off)
     bool ordered = false;
     uint* perm = nullptr;                  // device copy (npad)
+    uint* sort_tmp = nullptr;              // scratch of the upload's sort
     std::vector<uint> hperm;               // host copy (n), fetched on first use after an upload
     bool hperm_stale = false;              // the device copy is newer than hperm
     cudaEvent_t h2d_done = nullptr;        // a host upload's copies have read the caller's buffers

@@ -96,7 +96,7 @@ int RadixSort(KeyValuePair* pData0, KeyValuePair* pData1,
  * latency-critical loop that must not pay a first-call allocation): the same
  * stable sort and result, with its scratch in a fixed device array inside the
  * library instead of cudaMalloc'd memory.  At most 4,194,304 records (larger
- * requests return DEM_ERR_ARG); the array (about 2 MiB) is held on every GPU
+ * requests return DEM_ERR_ARG); the array (about 1 MiB) is held on every GPU
  * that loads the library until exit.  The first call on each device sets up
  * the array's address, which may also load the library's device code (and
  * with it reserve device memory) under CUDA's lazy module loading: make that
