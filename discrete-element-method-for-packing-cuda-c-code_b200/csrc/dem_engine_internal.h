@@ -367,6 +367,7 @@ struct dem_ctx {
     size_t npart = 0;                        // partials per slot: fpart + nblk (the free kernel's)
     unsigned long long* rmax_bits = nullptr;
     void* host_pinned = nullptr;     // mirror for scalars
+    void* raw_tail = nullptr;        // the observables' device part (dem_scalars_enqueue)
     // debug force record
     bool record = false;
     double* dbgF = nullptr;
