@@ -213,8 +213,12 @@ __global__ void k_scatter(long long n, const uint* __restrict__ key, const uint*
 }
 
 // Row candidates kept per particle by the candidate pass; longer rows are
-// filtered again by the fill.
-constexpr uint kScr = 8;
+// filtered again by the fill.  Rows up to kRow, else up to kScr, are sorted in
+// registers: a few per cent of a bed's rows are longer than kRow, so most
+// warps have one, and sorting it in global memory is what the warp waits for
+// (the reverse rows of a 500,000-sphere bed 142 -> 47 us, its fill 200 -> 172
+// us, with the second size).
+constexpr uint kScr = 16, kRow = 8;
 
 // ------------------------------------------------------------- outer list
 // The re-list searches candidates in an outer list: per particle every other
@@ -377,7 +381,7 @@ __global__ void k_outer_fill(long long n, const uint* __restrict__ sid2, const R
         uint* __restrict__ njli, uint* __restrict__ bflag, uint* __restrict__ scr
 #define DEM_FILTER_ARGS \
     n, S, R, g, skin, coff, cln, ccap, wslot, wlist, wcount, cc_parent, cc_zero, cc_base, np, ikey, njli, bflag, scr
-// The candidate pass for kFilterItems consecutive particles i0, i0+1, ...
+// The candidate pass for K consecutive particles i0, i0+1, ...
 // of one thread: their cell words (wall-candidacy bit) and outer-row bounds
 // are loaded together first, so that the thread waits on one chain of loads
 // rather than one per particle; only particles with outer candidates load
@@ -472,15 +476,22 @@ __device__ __forceinline__ FilterCounts<K> filter_items(long long i0, DEM_FILTER
 // (row offsets off, reverse-row offsets roff, bound positions bpos; totals
 // at [n]) by a single-pass scan with decoupled look-back (Merrill & Garland,
 // "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016): tiles
-// of kFilterTile particles (kFilterItems consecutive ones per thread) take
-// tickets in the order they start, publish
-// their totals, and add up the published words of the tiles before them, so
-// no tile waits on one that has not started.  The tile also writes the bound
+// of K consecutive particles per thread (filter_items_of) take tickets in the
+// order they start, publish their totals, and add up the published words of
+// the tiles before them, so no tile waits on one that has not started.  The tile also writes the bound
 // list (ascending id) and the free list.  Look-back words (lb): [0] the tile
 // ticket, then per tile and count a 64-bit word, the value in the low 32 bits
 // and the kind above (1: the tile's own total, 2: the total through the
 // tile); the fill clears them for the next re-list.
 constexpr int kFilterThreads = 512, kFilterItems = 4, kFilterTile = kFilterThreads * kFilterItems;
+// One particle per thread up to kFilterSmall of them: at four, 20,000 spheres
+// are ten tiles on ten SMs, and a bed's rows (~25 outer candidates each) one
+// after the other: 39 -> 12 us for a bed of 20,000, 45 -> 16 us of 100,000 in
+// FP64.  Five windows of a 200,000-sphere gas take 718 us with four and 708 us
+// with one; of 500,000 spheres 1,000 and 1,017 us.
+constexpr long long kFilterSmall = 1 << 18;
+inline int filter_items_of(long long n) { return n <= kFilterSmall ? 1 : kFilterItems; }
+inline long long filter_tiles(long long n) { return grid_for(n, kFilterThreads * filter_items_of(n)); }
 // limits and words of the bounded waits (grid_wait, tile_wait)
 constexpr unsigned long long kBarrierNs = 1000000000ull;   // 1 s
 constexpr uint kBarrierMinPolls = 200000u;                 // >= ~0.1 s of polling
@@ -498,7 +509,9 @@ __device__ __forceinline__ void wait_gave_up(EngineWords* w, uint site) {
 }
 // [0, 2 + 6 T) the candidate pass's words (T: its tiles of np particles),
 // then the component pass's: 2 + 2 Tc (Tc: its tiles of np entries)
-inline size_t lb_cc(long long np) { return 2 + 6 * (size_t)grid_for(np, kFilterTile); }
+inline size_t lb_cc(long long np) {   // the most tiles of any n <= np
+    return 2 + 6 * (size_t)std::max(grid_for(np, kFilterTile), grid_for(std::min(np, kFilterSmall), kFilterThreads));
+}
 inline size_t lb_words(long long np) { return lb_cc(np) + 2 + 2 * (size_t)grid_for(np, kCcThreads); }
 
 __device__ __forceinline__ void lb_store(unsigned long long* p, unsigned long long v) {
@@ -509,7 +522,7 @@ __device__ __forceinline__ unsigned long long lb_load(const unsigned long long* 
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-template <typename Real>
+template <typename Real, int K>
 __global__ void __launch_bounds__(kFilterThreads) k_filter_scan(DEM_FILTER_PARAMS, EngineWords* words, uint* lb,
                                                                 uint* __restrict__ off, uint* __restrict__ roff,
                                                                 uint* __restrict__ bpos, uint* __restrict__ blist,
@@ -529,19 +542,19 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_scan(DEM_FILTER_PARAM
         if (threadIdx.x == 0) wait_gave_up(words, kWaitFilterTicket);
         return;
     }
-    // the thread's kFilterItems consecutive particles
-    const long long i0 = (long long)tile * kFilterTile + (long long)threadIdx.x * kFilterItems;
+    // the thread's K consecutive particles
+    const long long i0 = ((long long)tile * kFilterThreads + threadIdx.x) * K;
     if (ccw) {   // the component pass's words and batch windows start empty
         const long long nthr = (long long)gridDim.x * kFilterThreads;
         const long long t0 = (long long)tile * kFilterThreads + threadIdx.x;
         if (t0 < 4) ccw[t0] = 0u;
         for (long long k = t0; k < 3 * nbb; k += nthr) bw[k] = k < nbb ? 0xffffffffu : 0u;
     }
-    const FilterCounts<kFilterItems> fc = filter_items<Real, kFilterItems>(i0, DEM_FILTER_ARGS);
+    const FilterCounts<K> fc = filter_items<Real, K>(i0, DEM_FILTER_ARGS);
     const uint *up = fc.up, *dn = fc.dn, *bd = fc.bd;
     uint v[3] = {0u, 0u, 0u}, mrow = 0;
 #pragma unroll
-    for (int k = 0; k < kFilterItems; k++) {
+    for (int k = 0; k < K; k++) {
         v[0] += up[k]; v[1] += dn[k]; v[2] += bd[k];
         mrow = max(mrow, up[k] + dn[k]);
     }
@@ -638,7 +651,7 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_scan(DEM_FILTER_PARAM
     uint e1 = s_pre[1] + s_w[1][warp] + inc[1] - v[1];
     uint e2 = s_pre[2] + s_w[2][warp] + inc[2] - v[2];
 #pragma unroll
-    for (int k = 0; k < kFilterItems; k++) {
+    for (int k = 0; k < K; k++) {
         const long long ii = i0 + k;
         if (ii < n) {
             const uint i = (uint)ii;
@@ -721,35 +734,43 @@ __device__ __forceinline__ bool dense_list(long long pairs, long long nb) { retu
         if (cc_parent && left_) cc_union(cc_parent, i, j); /* the window's components (cluster batches) */            \
     } while (0)
 
+template <int N, typename Real>
+__device__ __forceinline__ void fill_row(uint i, uint b, uint e, uint ob, uint oe, DEM_FILL_PARAMS) {
+    static_assert(N % 4 == 0 && N <= (int)kScr && kScr % 4 == 0, "16-byte words of candidates");
+    uint r[N], o[N];
+#pragma unroll
+    for (uint k = 0; k < N; k += 4) {
+        const uint4 w = reinterpret_cast<const uint4*>(scr + (size_t)i * kScr)[k / 4];
+        r[k] = w.x; r[k + 1] = w.y; r[k + 2] = w.z; r[k + 3] = w.w;
+    }
+#pragma unroll
+    for (uint k = 0; k < N; k++) {
+        if (k >= e - b) r[k] = kEmpty;
+        o[k] = k < oe - ob ? oln[ob + k] : kEmpty;
+    }
+    sort_regs(r);
+#pragma unroll
+    for (uint k = 0; k < N; k++) {
+        if (k >= e - b) continue;
+        const uint j = r[k];
+        uint lo = kEmpty;
+#pragma unroll
+        for (uint m = 0; m < N; m++)
+            if (o[m] == j) lo = ob + m;
+        ln[b + k] = j;
+        DEM_FILL_PAIR(b + k, j, lo);
+    }
+}
+
 template <typename Real> __device__ __forceinline__ void fill_item(uint i, DEM_FILL_PARAMS) {
     const uint b = off[i], e = off[i + 1];
     if (e == b) return;
     const bool old_ok = (long long)ooff[n] <= cap;   // an overflowed old list carries nothing
     const uint ob = old_ok ? ooff[i] : 0u, oe = old_ok ? ooff[i + 1] : 0u;
-    if (e - b <= kScr && oe - ob <= kScr) {   // the usual row: in registers, its loads side by side
-        static_assert(kScr == 8, "two 16-byte words of candidates");
-        uint r[kScr], o[kScr];
-        const uint4 r0 = reinterpret_cast<const uint4*>(scr)[2 * (size_t)i], r1 = reinterpret_cast<const uint4*>(scr)[2 * (size_t)i + 1];
-        r[0] = r0.x; r[1] = r0.y; r[2] = r0.z; r[3] = r0.w; r[4] = r1.x; r[5] = r1.y; r[6] = r1.z; r[7] = r1.w;
-#pragma unroll
-        for (uint k = 0; k < kScr; k++) {
-            if (k >= e - b) r[k] = kEmpty;
-            o[k] = k < oe - ob ? oln[ob + k] : kEmpty;
-        }
-        sort_regs(r);
-#pragma unroll
-        for (uint k = 0; k < kScr; k++) {
-            if (k >= e - b) continue;
-            const uint j = r[k];
-            uint lo = kEmpty;
-#pragma unroll
-            for (uint m = 0; m < kScr; m++)
-                if (o[m] == j) lo = ob + m;
-            ln[b + k] = j;
-            DEM_FILL_PAIR(b + k, j, lo);
-        }
-        return;
-    }
+    // in registers, the loads side by side: the usual row, and the long ones of a
+    // dense bed (where most warps have one)
+    if (e - b <= kRow && oe - ob <= kRow) return fill_row<kRow, Real>(i, b, e, ob, oe, DEM_FILL_ARGS);
+    if (e - b <= kScr && oe - ob <= kScr) return fill_row<kScr, Real>(i, b, e, ob, oe, DEM_FILL_ARGS);
     if (e - b <= kScr) {
         for (uint k = 0; k < e - b; k++) ln[b + k] = scr[(size_t)i * kScr + k];
     } else {   // a long row: filter the particle's outer row again
@@ -792,6 +813,20 @@ __global__ void k_nbr_fill(DEM_FILL_PARAMS, const uint* __restrict__ bpos, const
     for (long long t = tid; t < nb; t += nthr) fill_item<Real>(blist[t], DEM_FILL_ARGS);
 }
 
+template <int N>
+__device__ __forceinline__ void rev_row(uint b, uint e, uint* __restrict__ rk, uint* __restrict__ ru) {
+    uint r[N];
+#pragma unroll
+    for (uint k = 0; k < N; k++) r[k] = k < e - b ? rk[b + k] : kEmpty;
+    sort_regs(r);
+#pragma unroll
+    for (uint k = 0; k < N; k++)
+        if (k < e - b) {
+            rk[b + k] = r[k];
+            ru[r[k]] = b + k;
+        }
+}
+
 // Sort each reverse row (pair indices ascending: a deterministic order for
 // the gather) and record each pair's reverse slot ru[k]; every particle with
 // a reverse row is bound (the pass strides over the bound list).  With
@@ -812,17 +847,10 @@ __global__ void k_rev_sort(long long n, const uint* __restrict__ roff, uint* __r
          t += (long long)gridDim.x * blockDim.x) {
         const uint i = blist[t];
         const uint b = roff[i], e = roff[i + 1];
-        if (e - b <= kScr) {   // the usual row: in registers
-            uint r[kScr];
-#pragma unroll
-            for (uint k = 0; k < kScr; k++) r[k] = k < e - b ? rk[b + k] : kEmpty;
-            sort_regs(r);
-#pragma unroll
-            for (uint k = 0; k < kScr; k++)
-                if (k < e - b) {
-                    rk[b + k] = r[k];
-                    ru[r[k]] = b + k;
-                }
+        if (e - b <= kRow) {   // in registers: the usual row, and the long ones of a dense bed
+            rev_row<kRow>(b, e, rk, ru);
+        } else if (e - b <= kScr) {
+            rev_row<kScr>(b, e, rk, ru);
         } else {
             isort_u32(rk + b, e - b);
             for (uint u = b; u < e; u++) ru[rk[u]] = u;
@@ -2485,7 +2513,8 @@ template <typename Real> int launch_relist(dem_ctx* c, int src) {
     if (rc) return rc;
     const Real skin = (Real)c->cfg.skin;
     // candidates, their counts' scans, bound and free lists: one pass
-    k_filter_scan<Real><<<grid_for(n, kFilterTile), kFilterThreads, 0, s>>>(
+    const auto filter = filter_items_of(n) == 1 ? k_filter_scan<Real, 1> : k_filter_scan<Real, kFilterItems>;
+    filter<<<(unsigned)filter_tiles(n), kFilterThreads, 0, s>>>(
         n, S, (const Real*)c->rad, g, skin, (const uint*)c->coff, (const uint*)c->cln, c->ccap, c->wslot, c->wlist,
         c->wcount, cc ? c->cc_parent : nullptr, c->cc_size, c->cc_base, c->npad, (const uint*)c->ikey, c->njli,
         c->bflag, c->scr,

@@ -53,6 +53,7 @@ template <> struct TileCap<double> {
 constexpr uint kTileMin = 32;        // particles per tile at least (small systems)
 constexpr uint kTileNbr = 128;       // tiles that share pairs with one tile, at most
 constexpr uint kTileHash = 512;      // their hash set while they are collected
+constexpr uint kTileRow = 8;         // row entries that k_tile_lists holds in registers
 constexpr uint kFlagStride = 32;     // words between step counters: a 128-byte line each (in 14 shared lines the
                                      // polls of 436 tiles queued at a few L2 slices: ~4,800 cycles a wait)
 constexpr uint kCurveEvery = 256;    // windows between two computations of the curve: at 0.1 m/s a sphere of the
@@ -213,9 +214,12 @@ __device__ __forceinline__ uint curve_bin(const V3<double>& p, const GridC& g, c
 // block: its pairs (the rows of its particles, and the reverse-row pairs
 // whose lower particle is in another tile), the tables above, the wall items,
 // and its particles' states in tile order.  One launch: as separate kernels
-// the window graph took 24 more nodes, 90 us longer to instantiate.
+// the window graph took 24 more nodes, 90 us longer to instantiate.  Bound by
+// the latency of its gathers; with the partners' slots held in registers and
+// three blocks per SM (85 registers): 44 -> 31 us for a bed of 20,000 spheres,
+// 88 -> 65 us of 100,000 in FP64, 187 -> 158 us of 500,000.
 template <typename Real, bool PP>
-__global__ void __launch_bounds__(TileCap<Real>::P)
+__global__ void __launch_bounds__(TileCap<Real>::P, 3)
     k_tile_lists(StepArgs<Real> a, TileArgs<Real> T, const uint* __restrict__ bflag, GridC g, CurveGrid cg, uint ntmax,
                  uint* key, uint* __restrict__ arrival, uint* __restrict__ count, uint* __restrict__ start,
                  uint* __restrict__ bsum, uint* bar) {
@@ -337,8 +341,40 @@ __global__ void __launch_bounds__(TileCap<Real>::P)
             r0 = a.roff[id]; nr = a.roff[id + 1] - r0;
             if (!PP) ws = a.wslot[id];   // PP: a particle steps its walls itself
         }
-        for (uint e = 0; e < no; e++) ni += __ldcg(T.inv + a.ln[o0 + e]) - first < m ? 1u : 0u;   // unsigned: inside the tile
-        for (uint u = 0; u < nr; u++) nc += __ldcg(T.inv + a.lp[a.rk[r0 + u]]) - first < m ? 0u : 1u;
+        // the partners' slots of the first kTileRow entries, loaded side by side
+        // and kept: one after the other, a row's entries are a chain of loads
+        // (three for a reverse entry), and each of the three walks below had it
+        uint so[kTileRow], rr[kTileRow], rl[kTileRow], sr[kTileRow];
+#pragma unroll
+        for (uint e = 0; e < kTileRow; e++) {
+            so[e] = e < no ? a.ln[o0 + e] : kEmpty;
+            rr[e] = e < nr ? a.rk[r0 + e] : kEmpty;
+        }
+#pragma unroll
+        for (uint e = 0; e < kTileRow; e++) {
+            if (e < no) so[e] = __ldcg(T.inv + so[e]);
+            rl[e] = e < nr ? a.lp[rr[e]] : kEmpty;
+        }
+#pragma unroll
+        for (uint e = 0; e < kTileRow; e++) sr[e] = e < nr ? __ldcg(T.inv + rl[e]) : kEmpty;
+        // f(place in the row, slot) over the row; g(place, pair, lo, slot) over the reverse row
+        auto own = [&](auto&& f) {
+#pragma unroll
+            for (uint e = 0; e < kTileRow; e++)
+                if (e < no) f(e, so[e]);
+            for (uint e = kTileRow; e < no; e++) f(e, __ldcg(T.inv + a.ln[o0 + e]));
+        };
+        auto rev = [&](auto&& f) {
+#pragma unroll
+            for (uint e = 0; e < kTileRow; e++)
+                if (e < nr) f(e, rr[e], rl[e], sr[e]);
+            for (uint e = kTileRow; e < nr; e++) {
+                const uint k = a.rk[r0 + e], lo = a.lp[k];
+                f(e, k, lo, __ldcg(T.inv + lo));
+            }
+        };
+        own([&](uint, uint s) { ni += s - first < m ? 1u : 0u; });   // unsigned: inside the tile
+        rev([&](uint, uint, uint, uint s) { nc += s - first < m ? 0u : 1u; });
         for (uint k = p; k < kTileHash; k += kTileThreads) s_hash[k] = kEmpty;
         if (p == 0) s_nn = 0u;
         s_own[p] = no;
@@ -372,8 +408,8 @@ __global__ void __launch_bounds__(TileCap<Real>::P)
             }
             atomicAdd(&s_nn, kTileNbr);   // the set is full: too many
         };
-        for (uint e = 0; e < no; e++) meet(__ldcg(T.inv + a.ln[o0 + e]));
-        for (uint u = 0; u < nr; u++) meet(__ldcg(T.inv + a.lp[a.rk[r0 + u]]));
+        own([&](uint, uint s) { meet(s); });
+        rev([&](uint, uint, uint, uint s) { meet(s); });
         __syncthreads();
         const uint nnbr = s_nn;
         // whether it fits (the same for every thread): the arrays' strides, a
@@ -399,8 +435,8 @@ __global__ void __launch_bounds__(TileCap<Real>::P)
         uint4* tp = reinterpret_cast<uint4*>(B + L.op);
         uint* tk = T.tk + (size_t)t * Q;
         uint ii = s_ib[p], hh = s_hb[p];
-        for (uint e = 0; e < no; e++) {
-            const uint k = o0 + e, res = s_ob[p] + e, s = __ldcg(T.inv + a.ln[k]);
+        own([&](uint e, uint s) {
+            const uint k = o0 + e, res = s_ob[p] + e;
             if (s - first < m) {
                 te[ii] = p | ((s - first) << 9) | (res << 18);
                 tk[ii++] = k;
@@ -409,10 +445,9 @@ __global__ void __launch_bounds__(TileCap<Real>::P)
                 te[tin + hh] = p | (res << 18);
                 tk[tin + hh++] = k;
             }
-        }
+        });
         uint c = 0;
-        for (uint u = 0; u < nr; u++) {
-            const uint k = a.rk[r0 + u], lo = a.lp[k], s = __ldcg(T.inv + lo);
+        rev([&](uint u, uint k, uint lo, uint s) {
             uint res;
             if (s - first < m) {
                 res = s_ob[s - first] + (k - a.off[lo]);
@@ -423,7 +458,7 @@ __global__ void __launch_bounds__(TileCap<Real>::P)
                 tk[tin + hh++] = k | 0x80000000u;
             }
             tr[s_rb[p] + u] = (unsigned short)res;
-        }
+        });
         if (ws != kEmpty) T.twl[(size_t)t * PC + s_wb[p]] = (unsigned short)p;
         if (p < m) {
             tp[p] = make_uint4(s_ob[p] | (no << 16), s_rb[p] | (nr << 16), ws != kEmpty ? tot + s_wb[p] : kEmpty, id);
