@@ -1,9 +1,10 @@
 // dem_compat.cu -- the reference-compatible entry points (the extern "C"
 // wrapper set of particleSystem.cu:13-424) on sm_100a, FP64, reference data
-// layout (xyz-interleaved double arrays).  Kernels follow the reference's
-// decomposition -- one thread per particle for hash / neighbour rows / gather
-// / wall / update, one thread per candidate pair for the force -- with the
-// missing kernels and force laws written from their call contracts.
+// layout (xyz-interleaved double arrays).  The kernels: one thread per particle
+// for hash / gather / wall / update, a warp per particle for neighbour rows
+// and pairs (the reference: a thread), one thread per candidate
+// pair for the force -- with the missing kernels and force laws written from
+// their call contracts.
 #include <cstdio>
 #include <mutex>
 #include <vector>
@@ -102,15 +103,13 @@ __device__ __forceinline__ void isort(uint* a, uint len) {
     }
 }
 
-// neighborarrayD (called at particleSystem.cu:85; not in the reference):
-// 27-cell walk from i's cell, cell members from cellStart until the key
-// changes; candidate when |x_i - x_j|^2 < cub^2.
-__global__ void k_neighbor_array(int n, const double3* __restrict__ pos, const uint2* __restrict__ hash,
-                                 const uint* __restrict__ cellStart, uint3 gs, double3 cs, double3 o, int maxppc,
-                                 uint* __restrict__ Anei, uint* __restrict__ njgi, uint* __restrict__ njli,
-                                 uint* status) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// One particle's row by one thread, in two passes over the 27 cells: rows
+// longer than the warp's list below, and rows cut at their capacity (which
+// candidates stay follows the order of the cells).
+__device__ void neighbor_row_serial(int i, int n, const double3* __restrict__ pos, const uint2* __restrict__ hash,
+                                    const uint* __restrict__ cellStart, uint3 gs, double3 cs, double3 o, int maxppc,
+                                    uint* __restrict__ Anei, uint* __restrict__ njgi, uint* __restrict__ njli,
+                                    uint* status) {
     const double3 pi = pos[i];
     uint gx, gy, gz;
     ref_cell(pi, gs, cs, o, gx, gy, gz);
@@ -183,104 +182,231 @@ __global__ void k_neighbor_array(int n, const double3* __restrict__ pos, const u
     njli[i] = nlw;
 }
 
+// neighborarrayD (called at particleSystem.cu:85; not in the reference):
+// 27-cell walk from i's cell, cell members from cellStart until the key
+// changes; candidate when |x_i - x_j|^2 < cub^2.  A warp per particle, a lane
+// per cell: a cell's members are one dependent chain of loads (key, index,
+// position), and with a thread per particle 27 of them, twice, followed each
+// other.  The candidates collect in shared memory and each finds its place
+// in the row by counting the smaller ones (j > i first, then j < i, both
+// ascending).  The warp writes its whole row, the rest kEmpty.  50,000 spheres
+// of a bed, rows of 9.7: 88 -> 35 us.
+constexpr int kRowWarps = kBlock / 32, kRowList = 96;
+__global__ void __launch_bounds__(kBlock)
+    k_neighbor_array(int n, const double3* __restrict__ pos, const uint2* __restrict__ hash,
+                     const uint* __restrict__ cellStart, uint3 gs, double3 cs, double3 o, int maxppc,
+                     uint* __restrict__ Anei, uint* __restrict__ njgi, uint* __restrict__ njli, uint* status) {
+    __shared__ uint s_list[kRowWarps][kRowList];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * kRowWarps + warp;
+    if (i >= n) return;
+    uint* list = s_list[warp];
+    const double3 pi = pos[i];
+    uint gx, gy, gz;
+    ref_cell(pi, gs, cs, o, gx, gy, gz);
+    const double cub2 = c_cub * c_cub;
+    uint c = 0, t = kEmpty;
+    if (lane < 27) {
+        const int x = (int)gx + lane % 3 - 1, y = (int)gy + lane / 3 % 3 - 1, z = (int)gz + lane / 9 - 1;
+        if (x >= 0 && x < (int)gs.x && y >= 0 && y < (int)gs.y && z >= 0 && z < (int)gs.z) {
+            c = ((uint)z * gs.y + (uint)y) * gs.x + (uint)x;
+            t = cellStart[c];
+        }
+    }
+    uint cnt = 0;
+    // rounds: a lane's next member; the warp's new candidates are appended
+    bool open = t != kEmpty;
+    while (__any_sync(0xffffffffu, open)) {
+        bool take = false;
+        uint j = 0;
+        if (open) {
+            open = t < (uint)n;
+            if (open) {
+                const uint2 h = hash[t++];
+                open = h.x == c;
+                if (open && h.y != (uint)i) {
+                    j = h.y;
+                    const double3 pj = pos[j];
+                    const double ddx = pj.x - pi.x, ddy = pj.y - pi.y, ddz = pj.z - pi.z;
+                    take = ddx * ddx + ddy * ddy + ddz * ddz < cub2;
+                }
+            }
+        }
+        const uint m = __ballot_sync(0xffffffffu, take), at = cnt + __popc(m & ((1u << lane) - 1u));
+        if (take && at < (uint)kRowList) list[at] = j;
+        cnt += __popc(m);
+    }
+    uint* row = Anei + (size_t)i * maxppc;
+    if (cnt > (uint)kRowList || cnt > (uint)maxppc) {
+        for (uint s = lane; s < (uint)maxppc; s += 32) row[s] = kEmpty;
+        __syncwarp();
+        if (lane == 0)
+            neighbor_row_serial(i, n, pos, hash, cellStart, gs, cs, o, maxppc, Anei, njgi, njli, status);
+        return;
+    }
+    __syncwarp();
+    uint nu = 0;
+    for (uint s = lane; s < (uint)kRowList; s += 32) {
+        const uint mine = s < cnt ? list[s] : 0u;
+        // j > i before j < i: the difference j - i - 1 wraps for the lower
+        // ones, and keeps both ascending
+        const uint key = mine - (uint)i - 1u;
+        uint rank = 0;
+        for (uint u = 0; u < cnt; u++) {
+            const uint k = list[u] - (uint)i - 1u;
+            rank += k < key || (k == key && u < s);
+        }
+        if (s < cnt) row[rank] = mine;
+        nu += __popc(__ballot_sync(0xffffffffu, s < cnt && mine > (uint)i));
+        if ((s - lane) + 32 >= cnt) break;
+    }
+    for (uint s = cnt + lane; s < (uint)maxppc; s += 32) row[s] = kEmpty;
+    if (lane == 0) {
+        njgi[i] = nu;
+        njli[i] = cnt - nu;
+    }
+}
+
 // b[i] += a[i] (addTwoArraysD, neiglist.cu:122-130): exclusive -> inclusive scan.
 __global__ void k_add_two(uint* b, const uint* a, uint n) {
     uint i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) b[i] += a[i];
 }
 
-// pairlistD (called at particleSystem.cu:172; not in the reference).
-__global__ void k_pairlist(uint n, const uint* __restrict__ sjgi, const uint* __restrict__ oldsjgi,
-                           const uint* __restrict__ oldLn, const uint* __restrict__ Anei, const uint* __restrict__ njgi,
-                           const uint* __restrict__ njli, const double3* __restrict__ olddispt,
-                           const double* __restrict__ oldfricp, int maxppc, size_t capP, uint* __restrict__ Aref,
-                           uint* __restrict__ Lp, uint* __restrict__ Ln, double3* __restrict__ dispt,
-                           double* __restrict__ fricp) {
-    uint i = blockIdx.x * blockDim.x + threadIdx.x;
+// pairlistD (called at particleSystem.cu:172; not in the reference).  A warp
+// per particle, a lane per row entry: an entry searches its old row (or the
+// partner's row) by itself, and the lanes write the pairs side by side (a
+// thread per particle, 50,000 spheres, rows of 9.7: 23 -> 18 us).
+__global__ void __launch_bounds__(kBlock)
+    k_pairlist(uint n, const uint* __restrict__ sjgi, const uint* __restrict__ oldsjgi,
+               const uint* __restrict__ oldLn, const uint* __restrict__ Anei, const uint* __restrict__ njgi,
+               const uint* __restrict__ njli, const double3* __restrict__ olddispt,
+               const double* __restrict__ oldfricp, int maxppc, size_t capP, uint* __restrict__ Aref,
+               uint* __restrict__ Lp, uint* __restrict__ Ln, double3* __restrict__ dispt,
+               double* __restrict__ fricp) {
+    const uint i = blockIdx.x * kRowWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (i >= n) return;
-    const uint ngi = njgi[i];
+    const uint ngi = njgi[i], nt = ngi + njli[i];
     const uint base = sjgi[i] - ngi;
     uint os = i > 0 ? oldsjgi[i - 1] : 0u, oe = oldsjgi[i];
     if ((size_t)oe > capP) oe = (uint)capP;
     if (os > oe) os = oe;
     const uint* row = Anei + (size_t)i * maxppc;
     uint* aref = Aref + (size_t)i * maxppc;
-    for (uint s = 0; s < ngi; s++) {
-        const uint k = base + s, j = row[s];
-        if ((size_t)k >= capP) break;   // caller sized Lp/Ln below the list (maxCn < row length)
-        Lp[k] = i;
-        Ln[k] = j;
-        aref[s] = k;
-        double3 h = make_double3(0.0, 0.0, 0.0);
-        double fr = 0.0;
-        for (uint t = os; t < oe; t++) {
-            if (oldLn[t] == j) { h = olddispt[t]; fr = oldfricp[t]; break; }
-        }
-        dispt[k] = h;
-        fricp[k] = fr;
-    }
-    const uint nli = njli[i];
-    for (uint s = ngi; s < ngi + nli; s++) {
+    for (uint s = lane; s < nt; s += 32) {
         const uint j = row[s];
-        uint kk = kEmpty;
-        const uint* rowj = Anei + (size_t)j * maxppc;
-        const uint ngj = njgi[j];
-        for (uint t = 0; t < ngj; t++)
-            if (rowj[t] == i) { kk = sjgi[j] - ngj + t; break; }
-        aref[s] = kk;
+        if (s < ngi) {
+            const uint k = base + s;
+            if ((size_t)k >= capP) continue;   // caller sized Lp/Ln below the list (maxCn < row length)
+            Lp[k] = i;
+            Ln[k] = j;
+            aref[s] = k;
+            double3 h = make_double3(0.0, 0.0, 0.0);
+            double fr = 0.0;
+            for (uint t = os; t < oe; t++) {
+                if (oldLn[t] == j) { h = olddispt[t]; fr = oldfricp[t]; break; }
+            }
+            dispt[k] = h;
+            fricp[k] = fr;
+        } else {
+            uint kk = kEmpty;
+            const uint* rowj = Anei + (size_t)j * maxppc;
+            const uint ngj = njgi[j];
+            for (uint t = 0; t < ngj; t++)
+                if (rowj[t] == i) { kk = sjgi[j] - ngj + t; break; }
+            aref[s] = kk;
+        }
     }
 }
 
-// calculateforcepairD (neiglist.cu:156-233) with the contact law.
-__global__ void k_force_pair(uint total, const double3* __restrict__ pos, const double3* __restrict__ pdis,
-                             const double3* __restrict__ angv, const double* __restrict__ rad,
-                             const double* __restrict__ rmass, const uint* __restrict__ Lp, const uint* __restrict__ Ln,
-                             uint* __restrict__ oldLn, double3* __restrict__ dispt, double* __restrict__ fricp,
-                             double3* __restrict__ olddispt, double* __restrict__ oldfricp, double inv_dt,
-                             double3* __restrict__ forcepair, double3* __restrict__ torqpairi,
-                             double3* __restrict__ torqpairj, uint* __restrict__ contactpair) {
-    uint k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= total) return;
-    const uint i = Lp[k], j = Ln[k];
-    const double3 xi = pos[i], xj = pos[j];
-    const double ri = rad[i], rj = rad[j];
-    V3<double> D = mk(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z);
-    const double dist = sqrt(dot(D, D));
-    const double delta = (ri + rj) - dist;
-    double3 hin = dispt[k];
-    V3<double> h = mk(hin.x, hin.y, hin.z);
-    const double3 z3 = make_double3(0.0, 0.0, 0.0);
-    if (delta > 0.0 && dist > 0.0) {
-        const V3<double> n = mk(D.x / dist, D.y / dist, D.z / dist);
-        const double mi = rmass[i], mj = rmass[j];
-        const double rstar = ri * rj / (ri + rj), mstar = mi * mj / (mi + mj);
-        const double3 ai3 = angv[i], aj3 = angv[j], di3 = pdis[i], dj3 = pdis[j];
-        const V3<double> ai = mk(ai3.x, ai3.y, ai3.z), aj = mk(aj3.x, aj3.y, aj3.z);
-        const V3<double> U = mk(dj3.x - di3.x, dj3.y - di3.y, dj3.z - di3.z) - cross(ri * ai + rj * aj, n);
-        V3<double> Fi, Ft, Mr;
-        contact_law<double>(delta, n, rstar, mstar, U, ai - aj, h, inv_dt, c_pp, Fi, Ft, Mr);
-        const V3<double> nxf = cross(n, Ft);
-        const V3<double> Ti = ri * nxf + Mr, Tj = rj * nxf - Mr;
-        const double fr = sqrt(dot(Ft, Ft));
-        forcepair[k] = make_double3(Fi.x, Fi.y, Fi.z);
-        torqpairi[k] = make_double3(Ti.x, Ti.y, Ti.z);
-        torqpairj[k] = make_double3(Tj.x, Tj.y, Tj.z);
-        dispt[k] = make_double3(h.x, h.y, h.z);
-        fricp[k] = fr;
-        contactpair[k] = 1u;
-        olddispt[k] = make_double3(h.x, h.y, h.z);
-        oldfricp[k] = fr;
-    } else {
-        forcepair[k] = z3;
-        torqpairi[k] = z3;
-        torqpairj[k] = z3;
-        dispt[k] = z3;
-        fricp[k] = 0.0;
-        contactpair[k] = 0u;
-        olddispt[k] = z3;
-        oldfricp[k] = 0.0;
+// A warp's 32 rows of three doubles, written as 96 consecutive doubles: a
+// lane's own row is three stores at a stride of 24 bytes, each of which touches
+// every sector of the warp's rows.  Doubles, not wider words: the caller's
+// arrays are aligned to 8 bytes only.
+__device__ __forceinline__ void store_rows(double* s, double* __restrict__ out, uint k0, uint total,
+                                           V3<double> v, double* __restrict__ out2 = nullptr) {
+    const uint lane = threadIdx.x & 31;
+    s[3 * lane] = v.x;
+    s[3 * lane + 1] = v.y;
+    s[3 * lane + 2] = v.z;
+    __syncwarp();
+#pragma unroll
+    for (uint e = 0; e < 3; e++) {
+        const uint w = e * 32 + lane;
+        if (w < 3 * min(total - k0, 32u)) {
+            const double d = s[w];
+            out[(size_t)k0 * 3 + w] = d;
+            if (out2) out2[(size_t)k0 * 3 + w] = d;
+        }
     }
-    oldLn[k] = j;
+    __syncwarp();
+}
+
+// calculateforcepairD (neiglist.cu:156-233) with the contact law: its quotients
+// and roots in the branch-free form where all are in range, else the library's
+// (the same bits).  Bound by the ~144 bytes a pair that the interface has it
+// write; 242,000 listed pairs, 149,000 touching: 20.5 -> 14.3 us.
+__global__ void __launch_bounds__(kBlock)
+    k_force_pair(uint total, const double3* __restrict__ pos, const double3* __restrict__ pdis,
+                 const double3* __restrict__ angv, const double* __restrict__ rad,
+                 const double* __restrict__ rmass, const uint* __restrict__ Lp, const uint* __restrict__ Ln,
+                 uint* __restrict__ oldLn, double* __restrict__ dispt, double* __restrict__ fricp,
+                 double* __restrict__ olddispt, double* __restrict__ oldfricp, double inv_dt,
+                 double* __restrict__ forcepair, double* __restrict__ torqpairi,
+                 double* __restrict__ torqpairj, uint* __restrict__ contactpair) {
+    __shared__ double s_row[kRowWarps][96];
+    const uint k0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u, k = k0 + (threadIdx.x & 31);
+    if (k0 >= total) return;
+    double* s = s_row[threadIdx.x >> 5];
+    V3<double> Fi = zero3<double>(), Ti = Fi, Tj = Fi, h = Fi;
+    double fr = 0.0;
+    uint hit = 0, j = 0;
+    if (k < total) {
+        const uint i = Lp[k];
+        j = Ln[k];
+        const double3 xi = pos[i], xj = pos[j];
+        const double ri = rad[i], rj = rad[j];
+        const V3<double> D = mk(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z);
+        const double d2 = dot(D, D), dist = sqrt(d2);
+        const double delta = (ri + rj) - dist;
+        if (delta > 0.0 && dist > 0.0) {
+            const V3<double> h0 = mk(dispt[(size_t)k * 3], dispt[(size_t)k * 3 + 1], dispt[(size_t)k * 3 + 2]);
+            const double mi = rmass[i], mj = rmass[j];
+            const double rr = ri * rj, mm = mi * mj;
+            const double3 ai3 = angv[i], aj3 = angv[j], di3 = pdis[i], dj3 = pdis[j];
+            const V3<double> ai = mk(ai3.x, ai3.y, ai3.z), aj = mk(aj3.x, aj3.y, aj3.z);
+            const V3<double> dd = mk(dj3.x - di3.x, dj3.y - di3.y, dj3.z - di3.z), ra = ri * ai + rj * aj;
+            V3<double> n, Ft, Mr;
+            bool ok = false;
+            h = h0;
+            if (c_pp.fast && x_mid(dist) && x_in(rr) && x_in(mm) && x_mid(ri + rj) && x_mid(mi + mj) &&
+                x_in(fabs(D.x)) && x_in(fabs(D.y)) && x_in(fabs(D.z))) {
+                n = mk(x_div(D.x, dist), x_div(D.y, dist), x_div(D.z, dist));
+                ok = contact_law_fast<double>(delta, n, x_div(rr, ri + rj), x_div(mm, mi + mj), dd - cross(ra, n),
+                                              ai - aj, h, inv_dt, c_pp, Fi, Ft, Mr);
+            }
+            if (!ok) {
+                n = mk(D.x / dist, D.y / dist, D.z / dist);
+                h = h0;
+                contact_law<double>(delta, n, rr / (ri + rj), mm / (mi + mj), dd - cross(ra, n), ai - aj, h, inv_dt,
+                                    c_pp, Fi, Ft, Mr);
+            }
+            const V3<double> nxf = cross(n, Ft);
+            Ti = ri * nxf + Mr;
+            Tj = rj * nxf - Mr;
+            fr = sqrt(dot(Ft, Ft));
+            hit = 1;
+        }
+        contactpair[k] = hit;
+        fricp[k] = fr;
+        oldfricp[k] = fr;
+        oldLn[k] = j;
+    }
+    __syncwarp();
+    store_rows(s, forcepair, k0, total, Fi);
+    store_rows(s, torqpairi, k0, total, Ti);
+    store_rows(s, torqpairj, k0, total, Tj);
+    store_rows(s, dispt, k0, total, h, olddispt);
 }
 
 // sumallforceiD (called at particleSystem.cu:262; not in the reference).
@@ -295,18 +421,28 @@ __global__ void k_sum_force(int n, int maxppc, const uint* __restrict__ njgi, co
     uint cnt = 0;
     const uint ng = njgi[i], nt = ng + njli[i];
     const uint* row = Aref + (size_t)i * maxppc;
-    for (uint s = 0; s < nt; s++) {
-        const uint k = row[s];
-        if (k == kEmpty) continue;
-        const double3 f = forcepair[k];
-        if (s < ng) {
-            const double3 t = torqpairi[k];
-            fx += f.x; fy += f.y; fz += f.z; tx += t.x; ty += t.y; tz += t.z;
-        } else {
-            const double3 t = torqpairj[k];
-            fx -= f.x; fy -= f.y; fz -= f.z; tx += t.x; ty += t.y; tz += t.z;
-        }
-        cnt += contactpair[k];
+    // four entries are loaded side by side and added in row order (50,000
+    // spheres, rows of 9.7: 14.3 -> 12.0 us; bound by the gathers' sectors)
+    for (uint s0 = 0; s0 < nt; s0 += 4) {
+        uint k[4], hit[4];
+        double3 f[4], t[4];
+#pragma unroll
+        for (uint e = 0; e < 4; e++) k[e] = s0 + e < nt ? row[s0 + e] : kEmpty;
+#pragma unroll
+        for (uint e = 0; e < 4; e++)
+            if (k[e] != kEmpty) {
+                f[e] = forcepair[k[e]];
+                t[e] = s0 + e < ng ? torqpairi[k[e]] : torqpairj[k[e]];
+                hit[e] = contactpair[k[e]];
+            }
+#pragma unroll
+        for (uint e = 0; e < 4; e++)
+            if (k[e] != kEmpty) {
+                if (s0 + e < ng) { fx += f[e].x; fy += f[e].y; fz += f[e].z; }
+                else { fx -= f[e].x; fy -= f[e].y; fz -= f[e].z; }
+                tx += t[e].x; ty += t[e].y; tz += t[e].z;
+                cnt += hit[e];
+            }
     }
     forcei[i] = make_double3(fx, fy, fz);
     torquei[i] = make_double3(tx, ty, tz);
@@ -351,11 +487,13 @@ __global__ void k_force_wall(int n, double3 ws, const double3* __restrict__ pos,
 // updatepositionD (neiglist.cu:308-409), adamp = bdamp = 1.  The block
 // maxima of the reference (partials reduced on the host) become one atomic
 // per block into device words: iall and the bit pattern of max(0, max z)
-// (non-negative doubles order like their bit patterns).
+// (non-negative doubles order like their bit patterns).  The last block hands
+// the words to the caller's pinned ones and clears them for the next call:
+// two fills and a copy less a step.
 __global__ void k_update(int n, double3* __restrict__ pos, double3* __restrict__ pdis, double3* __restrict__ angv,
                          const double* __restrict__ rmass, const double* __restrict__ inert,
                          const double3* __restrict__ forcei, const double3* __restrict__ torquei,
-                         double3* __restrict__ qi, double dt, uint* words) {
+                         double3* __restrict__ qi, double dt, uint* words, uint* host) {
     __shared__ unsigned long long smz[kBlock / 32];
     __shared__ uint sall[kBlock / 32];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -396,6 +534,15 @@ __global__ void k_update(int n, double3* __restrict__ pos, double3* __restrict__
         if (flag & 1u) atomicOr(&words[1], 1u);
         if (flag & 2u) atomicOr(&words[0], kStatusNonfinite);
         if (mb) atomicMax(reinterpret_cast<unsigned long long*>(&words[4]), mb);
+        __threadfence();
+        if (atomicAdd(&words[6], 1u) == gridDim.x - 1) {   // every block's part is in
+            __threadfence();
+            host[0] = atomicExch(&words[0], 0u);
+            host[1] = atomicExch(&words[1], 0u);
+            *reinterpret_cast<unsigned long long*>(host + 4) =
+                atomicExch(reinterpret_cast<unsigned long long*>(&words[4]), 0ull);
+            words[6] = 0;
+        }
     }
 }
 
@@ -487,8 +634,7 @@ int neighborarray(double* pos, unsigned int* particleHash, unsigned int* cellSta
     CompatDevice* cd;
     int rc = compat_device(&cd);
     if (rc) return rc;
-    DEM_CUDA_TRY(cudaMemsetAsync(Anei, 0xff, (size_t)numBodies * maxParticlesPerCell * sizeof(uint), g_stream));
-    k_neighbor_array<<<grid_for(numBodies, kBlock), kBlock, 0, g_stream>>>(
+    k_neighbor_array<<<grid_for(numBodies, kRowWarps), kBlock, 0, g_stream>>>(
         numBodies, (const double3*)pos, (const uint2*)particleHash, cellStart,
         make_uint3(gridSize[0], gridSize[1], gridSize[2]), d3(cellSize), d3(worldOrigin), maxParticlesPerCell, Anei,
         njgi, njli, cd->words);
@@ -538,7 +684,7 @@ int pairlist(unsigned int* sjgi, unsigned int* oldsjgi, unsigned int* oldLn, uns
     DEM_CUDA_TRY(cudaMemsetAsync(Ln, 0xff, capP * sizeof(uint), g_stream));
     DEM_CUDA_TRY(cudaMemsetAsync(dispt, 0, capP * 3 * sizeof(double), g_stream));
     DEM_CUDA_TRY(cudaMemsetAsync(fricp, 0, capP * sizeof(double), g_stream));
-    k_pairlist<<<grid_for(numBodies, kBlock), kBlock, 0, g_stream>>>(
+    k_pairlist<<<grid_for(numBodies, kRowWarps), kBlock, 0, g_stream>>>(
         numBodies, sjgi, oldsjgi, oldLn, Anei, njgi, njli, (const double3*)olddispt, oldfricp, maxParticlesPerCell,
         capP, Aref, Lp, Ln, (double3*)dispt, fricp);
     DEM_LAUNCH_CHECK();
@@ -555,8 +701,7 @@ int calculateforcepair(double* pos, double* pdis, double* angv, double* rad, dou
         return fail(DEM_ERR_ARG, "calculateforcepair: bad argument");
     k_force_pair<<<grid_for(totalcontacts, kBlock), kBlock, 0, g_stream>>>(
         totalcontacts, (const double3*)pos, (const double3*)pdis, (const double3*)angv, rad, rmass, Lp, Ln, oldLn,
-        (double3*)dispt, fricp, (double3*)olddispt, oldfricp, 1.0 / dt, (double3*)forcepair, (double3*)torqpairi,
-        (double3*)torqpairj, contactpair);
+        dispt, fricp, olddispt, oldfricp, 1.0 / dt, forcepair, torqpairi, torqpairj, contactpair);
     DEM_LAUNCH_CHECK();
     return DEM_OK;
 }
@@ -602,13 +747,10 @@ int updateposition(double worldSize[3], int numBodies, double* pos, double* pdis
     CompatDevice* cd;
     int rc = compat_device(&cd);
     if (rc) return rc;
-    DEM_CUDA_TRY(cudaMemsetAsync(cd->words + 1, 0, sizeof(uint), g_stream));
-    DEM_CUDA_TRY(cudaMemsetAsync(cd->words + 4, 0, 2 * sizeof(uint), g_stream));
     k_update<<<grid_for(numBodies, kBlock), kBlock, 0, g_stream>>>(
         numBodies, (double3*)pos, (double3*)pdis, (double3*)angv, rmass, inert, (const double3*)forcei,
-        (const double3*)torquei, (double3*)qi, dt, cd->words);
+        (const double3*)torquei, (double3*)qi, dt, cd->words, cd->host_words);
     DEM_LAUNCH_CHECK();
-    DEM_CUDA_TRY(cudaMemcpyAsync(cd->host_words, cd->words, 8 * sizeof(uint), cudaMemcpyDeviceToHost, g_stream));
     DEM_CUDA_TRY(cudaStreamSynchronize(g_stream));
     *iall = cd->host_words[1];
     unsigned long long mb;
@@ -616,10 +758,8 @@ int updateposition(double worldSize[3], int numBodies, double* pos, double* pdis
     double mz;
     memcpy(&mz, &mb, sizeof(mz));
     *maxhz = mz;
-    if (cd->host_words[0] & kStatusNonfinite) {
-        DEM_CUDA_TRY(cudaMemsetAsync(cd->words, 0, sizeof(uint), g_stream));
+    if (cd->host_words[0] & kStatusNonfinite)
         return fail(DEM_ERR_NONFINITE, "updateposition: non-finite position");
-    }
     return DEM_OK;
 }
 

@@ -9,10 +9,11 @@ namespace dem {
 
 struct CompatDevice {
     int device = -1;
-    uint* words = nullptr;           // device: [0] status bits, [1] iall, [2] pcntot, [4..5] maxhz bits (u64)
+    uint* words = nullptr;           // device: [0] status bits, [1] iall, [2] pcntot, [4..5] maxhz bits (u64),
+                                     // [6] blocks done
     uint* scratch = nullptr;         // device scratch
     size_t scratch_words = 0;
-    uint* host_words = nullptr;      // pinned mirror of words (8 uint)
+    uint* host_words = nullptr;      // pinned mirror of words
 };
 
 int compat_device(CompatDevice** out);
