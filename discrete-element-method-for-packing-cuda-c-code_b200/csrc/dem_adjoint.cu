@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 #include "dem_engine_internal.h"
 #include "dem_law_adj.cuh"
@@ -40,7 +41,13 @@ namespace {
 constexpr int kB = 256;
 constexpr int kPairB = 32;    // block size of k_adj_step; pbar holds one 12-slot row per block
 constexpr int kAB = 128;      // block size of k_adj_pairs and k_adj_bound
-constexpr int kPC = 20;       // doubles per pair of the two-phase reverse step's shares
+constexpr int kBG = 8;        // lanes per bound particle in k_adj_bound
+constexpr int kAC = 4;        // items per thread that k_adj_pairs sorts at a time
+// A share of the two-phase reverse step: the adjoints that a pair (a particle's
+// walls) sends to a particle -- x, d, a (3 each), radius, then whether the
+// share holds this step's values -- as three 32-byte words.  A pair slot has
+// two of them, lo's and hi's.
+constexpr int kShare = 12;
 constexpr long long kScatterPrime = 2654435761ll;
 
 struct Ck {
@@ -116,10 +123,8 @@ struct AdjWork {
     double *Xb = nullptr, *Db = nullptr, *Ab = nullptr, *Wb = nullptr, *Rb = nullptr;
     double* Hb[2] = {nullptr, nullptr};
     double* pbar = nullptr;      // npb x 12 (one row per reverse-step block: pair params 0-5, wall params 6-11)
-    double* PC = nullptr;        // kPC per pair slot: the shares a pair's reverse sends to lo and hi
-    uint* pon = nullptr;         // per pair slot: 1 if PC holds this step's shares
-    double* WS = nullptr;        // 10 per particle: its walls' shares (pair phase)
-    uint* wson = nullptr;        // per particle: 1 if WS holds this step's shares
+    double* PC = nullptr;        // two shares per pair slot: what a pair's reverse sends to lo and hi
+    double* WS = nullptr;        // a share per particle: its walls' (pair phase)
     unsigned grid_pairs = 1, grid_bound = 1;   // blocks of k_adj_pairs / k_adj_bound
     bool pair_parallel = true;   // two-phase reverse step (DEM_B200_ADJ=pp: k_adj_step)
     double* objp = nullptr;      // 3 per k_obj_potential block: energy, d/d estar (pair, wall)
@@ -188,8 +193,8 @@ int ensure_work(dem_ctx* c, long long seg, long long nck) {
         if ((rc = adj_grids(c))) return rc;
         w->npb = std::max<long long>(grid_for(c->n, kPairB), std::max(w->grid_pairs, w->grid_bound));
         if ((rc = dalloc(&w->pbar, (size_t)w->npb * 12))) return rc;
-        if (w->pair_parallel && ((rc = dalloc(&w->PC, (size_t)kPC * cap)) || (rc = dalloc(&w->pon, cap)) ||
-                                 (rc = dalloc(&w->WS, 10 * (size_t)np)) || (rc = dalloc(&w->wson, np))))
+        if (w->pair_parallel && ((rc = dalloc(&w->PC, 2 * (size_t)kShare * cap)) ||
+                                 (rc = dalloc(&w->WS, kShare * (size_t)np))))
             return rc;
         w->Xb = w->Xb2[0];
         w->Db = w->Db2[0];
@@ -516,20 +521,32 @@ __global__ void __launch_bounds__(kPairB) k_adj_step(
 // One reversed step of the bound particles in two pair-parallel phases (the
 // default; k_adj_step above is the particle-parallel form, DEM_B200_ADJ=pp).
 //
-// Phase A (k_adj_pairs), one thread per listed pair (lo, hi): the pair law is
-// evaluated forward from the tape and reversed once, with the force adjoint
-// of each side taken from the after-step state adjoints (the first half of
-// the integrator reverse); the pair's input-history adjoint goes to Hin, its
+// Phase A (k_adj_pairs): the law of each touching pair (lo, hi) is evaluated
+// forward from the tape and reversed once, with the force adjoint of each
+// side taken from the after-step state adjoints (the first half of the
+// integrator reverse); the pair's input-history adjoint goes to Hin, its
 // parameter adjoints into this block's row of pbar (slots 0-5), and the
-// adjoints it sends to lo and hi into PC (kPC doubles per pair: lo's x, d, a
-// and radius, then hi's), with pon[k] = 1.  A pair whose two spheres had no
-// pair contact in the forward step (taped count 0 on either side) only clears
-// its history adjoint.  Phase B (k_adj_bound), one thread per bound particle:
-// the integrator reverse, the sum of its pairs' shares (own row, then reverse
-// row, in list order: deterministic), the walls (parameter adjoints into
-// slots 6-11 of its block's row), and the state adjoints before the step.
-// The chain of one thread is one pair's law instead of all of a sphere's
-// pairs twice over; no atomics.
+// adjoints it sends to lo and hi into its two shares.  A block first sorts its
+// listed pairs into those that touch and the others (which only clear their
+// history adjoint and their shares' flags, as does a pair one of whose spheres
+// had no pair contact in the forward step), then gives every thread one that
+// touches: a law and its reverse are one chain of ~1,000 instructions, for
+// which a warp with half its lanes idle waits just as long.  The branch-free
+// quotients and roots (MathFast) shorten that chain; a pair out of their range
+// is done again with the library's.  A sixteenth of the blocks reverse the
+// bound particles' walls instead (slots 6-11, shares in WS): few particles
+// touch one, and among the pairs their chains were the last to end.
+//
+// Phase B (k_adj_bound), kBG lanes per bound particle: the integrator reverse
+// and the sum of its pairs' shares (lane l the l-th, l+kBG-th ... of its own
+// row and then of its reverse row, then the lanes in a tree: deterministic)
+// and its walls' -- the state adjoints before the step.  No atomics.
+//
+// Both are bound by latency, not by the FP64 pipe (9 %) or memory: phase A
+// runs at 255 registers, two blocks per SM (three, at 168, spill more than
+// they hide: 26 -> 31 us a step).  The tape of the step to be reversed next is
+// brought into L2 meanwhile.  A reversed step of 20,011 bed spheres (69,800
+// listed pairs): 49 -> 26 us (phase A 31 -> 21, phase B 18 -> 5).
 __device__ __forceinline__ void block_sum6(const double v[6], double* row) {
     __shared__ double sp[6][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -549,105 +566,209 @@ __device__ __forceinline__ void block_sum6(const double v[6], double* row) {
     __syncthreads();   // sp may be reused by the next call
 }
 
-template <typename Real>
-__global__ void __launch_bounds__(kAB) k_adj_pairs(
-    long long n, long long np, long long cap, AdjList L, const double* __restrict__ tx, const double* __restrict__ td,
-    const Real* __restrict__ ta, const double* __restrict__ th, const uint* __restrict__ tc, const Real* __restrict__ R,
-    LawParams<double> pp, double dt, double density, const double* __restrict__ Hout, double* __restrict__ Hin,
-    const double* __restrict__ Xa, const double* __restrict__ Da, const double* __restrict__ Aa,
-    double* __restrict__ PC, uint* __restrict__ pon, double* __restrict__ pbar, const uint* __restrict__ blist,
-    const uint* __restrict__ nbp, const double* __restrict__ twh, LawParams<double> pw, double hx, double hy,
-    double* __restrict__ WS, uint* __restrict__ wson, double* __restrict__ Wb) {
-    const double inv_dt = 1.0 / dt;
-    LawBar bp, bw;
-    lawbar_zero(bp);
-    lawbar_zero(bw);
-    // the list and the tape (the recompute's) may be read before the wait;
-    // the state and history adjoints are the predecessors'
-    const uint total = L.off[n];
-    const long long nb = (long long)*nbp;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const long long npr = (long long)total <= cap ? (long long)total : 0ll;
-    pdl_wait();
-    pdl_trigger();
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < npr + nb; k += stride) {
-        if (k >= npr) {
-            // a bound particle's walls: their VJP needs only the particle's
-            // force adjoints, so it runs beside the pairs; its shares go to
-            // WS for the particle phase, its history adjoint to Wb
-            const uint i = blist[k - npr];
-            V3d fbi, tbi;
-            partner_fb<Real>(R[i], np, i, dt, density, Xa, Da, Aa, fbi, tbi);
-            V3d xw = zero3<double>(), dw = zero3<double>(), aw = zero3<double>(), hwb = zero3<double>();
-            double rw = 0.0;
-            const int hit = wall_vjp(hx, hy, ld3(tx, np, i), ld3(td, np, i), ldA<Real>(ta, np, i), (double)R[i],
-                                     density, ld3(twh, np, i), pw, inv_dt, fbi, tbi, ld3(Wb, np, i), xw, dw, aw, rw,
-                                     hwb, bw);
-            st3(Wb, np, i, hwb);
-            if (hit) {
-                double* c = WS + 10 * (size_t)i;
-                c[0] = xw.x; c[1] = xw.y; c[2] = xw.z; c[3] = dw.x; c[4] = dw.y; c[5] = dw.z;
-                c[6] = aw.x; c[7] = aw.y; c[8] = aw.z; c[9] = rw;
-            }
-            wson[i] = hit ? 1u : 0u;
-            continue;
-        }
-        {
-            const uint lo = L.lp[k], hi = L.ln[k];
-            bool on = tc[lo] != 0 && tc[hi] != 0;
-            PairTape t;
-            if (on) {
-                const V3d hin = mk(th[k], th[cap + k], th[2 * cap + k]);
-                V3d Fi, Ti, Tj, ho;
-                on = pair_fwd(ld3(tx, np, lo), ld3(tx, np, hi), ld3(td, np, lo), ld3(td, np, hi), ldA<Real>(ta, np, lo),
-                              ldA<Real>(ta, np, hi), (double)R[lo], (double)R[hi], hin, pp, inv_dt, density, t, Fi,
-                              Ti, Tj, ho) != 0;
-            }
-            if (!on) {
-                Hin[k] = 0.0; Hin[cap + k] = 0.0; Hin[2 * cap + k] = 0.0;
-                pon[k] = 0u;
-                continue;
-            }
-            V3d fbl, tbl, fbh, tbh;
-            partner_fb<Real>(R[lo], np, lo, dt, density, Xa, Da, Aa, fbl, tbl);
-            partner_fb<Real>(R[hi], np, hi, dt, density, Xa, Da, Aa, fbh, tbh);
-            V3d xl = zero3<double>(), xh = zero3<double>(), dl = zero3<double>(), dh = zero3<double>(),
-                al = zero3<double>(), ah = zero3<double>(), hinb = zero3<double>();
-            double rl = 0.0, rh = 0.0;
-            pair_rev(t, pp, inv_dt, density, fbl - fbh, tbl, tbh, mk(Hout[k], Hout[cap + k], Hout[2 * cap + k]), xl, xh,
-                     dl, dh, al, ah, rl, rh, hinb, bp);
-            Hin[k] = hinb.x; Hin[cap + k] = hinb.y; Hin[2 * cap + k] = hinb.z;
-            double* c = PC + (size_t)kPC * k;
-            c[0] = xl.x; c[1] = xl.y; c[2] = xl.z; c[3] = dl.x; c[4] = dl.y; c[5] = dl.z;
-            c[6] = al.x; c[7] = al.y; c[8] = al.z; c[9] = rl;
-            c[10] = xh.x; c[11] = xh.y; c[12] = xh.z; c[13] = dh.x; c[14] = dh.y; c[15] = dh.z;
-            c[16] = ah.x; c[17] = ah.y; c[18] = ah.z; c[19] = rh;
-            pon[k] = 1u;
-        }
+// One of two shares, or a flag that it holds nothing.
+__device__ __forceinline__ void st_share(double* s, V3d x, V3d d, V3d a, double r) {
+    st32(s, x.x, x.y, x.z, d.x);
+    st32(s + 4, d.y, d.z, a.x, a.y);
+    st32(s + 8, a.z, r, 1.0, 0.0);
+}
+__device__ __forceinline__ void no_share(double* s) { s[10] = 0.0; }
+__device__ __forceinline__ void add_share(const double* s, V3d& xb, V3d& db, V3d& ab, double& rb) {
+    const Words4 u = ld32<false>(s), v = ld32<false>(s + 4), w = ld32<false>(s + 8);
+    if (w.c != 0.0) {
+        xb += mk(u.a, u.b, u.c);
+        db += mk(u.d, v.a, v.b);
+        ab += mk(v.c, v.d, w.a);
+        rb += w.b;
     }
-    const double v[6] = {bp.estar, bp.mu, bp.cn, bp.ct, bp.roll, bp.roll_rel};
-    block_sum6(v, pbar + (size_t)blockIdx.x * 12);
-    const double vw[6] = {bw.estar, bw.mu, bw.cn, bw.ct, bw.roll, bw.roll_rel};
-    block_sum6(vw, pbar + (size_t)blockIdx.x * 12 + 6);
 }
 
-__device__ __forceinline__ void add_share(const double* __restrict__ c, V3d& xb, V3d& db, V3d& ab, double& rb) {
-    xb += mk(c[0], c[1], c[2]);
-    db += mk(c[3], c[4], c[5]);
-    ab += mk(c[6], c[7], c[8]);
-    rb += c[9];
+// L2 prefetch of words p[0, count), the grid's threads side by side.
+template <typename T> __device__ __forceinline__ void prefetch_range(const T* p, long long count) {
+    const long long lines = (count * (long long)sizeof(T) + 127) / 128;
+    for (long long l = (long long)blockIdx.x * blockDim.x + threadIdx.x; l < lines;
+         l += (long long)gridDim.x * blockDim.x)
+        prefetch_l2(reinterpret_cast<const char*>(p) + 128 * l);
+}
+
+// What k_adj_pairs works on: a step's list, tape and adjoints.
+template <typename Real> struct AdjPairs {
+    long long n, np, cap;
+    AdjList L;
+    const double *tx, *td;
+    const Real* ta;
+    const double* th;
+    const uint* tc;
+    const Real* R;
+    LawParams<double> pp, pw;
+    double dt, density, hx, hy;
+    const double* Hout;
+    double* Hin;
+    const double *Xa, *Da, *Aa;
+    double *PC, *WS, *Wb, *pbar;
+    const uint *blist, *nb;
+    const double *twh, *tF, *tT;
+    int earlier;   // the tape holds the step before this one
+};
+
+// A touching pair's reverse; false, with nothing written, when a quotient or
+// root is out of MathFast's range.
+template <class M, typename Real>
+__device__ __forceinline__ bool adj_pair(const AdjPairs<Real>& a, long long k, LawBar& bp) {
+    const long long np = a.np, cap = a.cap;
+    const double inv_dt = 1.0 / a.dt;
+    const uint lo = a.L.lp[k], hi = a.L.ln[k];
+    const V3d hin = mk(a.th[k], a.th[cap + k], a.th[2 * cap + k]);
+    PairTape t;
+    V3d Fi, Ti, Tj, ho;
+    pair_fwd<M>(ld3(a.tx, np, lo), ld3(a.tx, np, hi), ld3(a.td, np, lo), ld3(a.td, np, hi), ldA<Real>(a.ta, np, lo),
+                ldA<Real>(a.ta, np, hi), (double)a.R[lo], (double)a.R[hi], hin, a.pp, inv_dt, a.density, t, Fi, Ti, Tj,
+                ho);
+    if (std::is_same<M, MathFast>::value && !(t.on && pair_in_range(t, a.pp))) return false;
+    V3d fbl, tbl, fbh, tbh;
+    partner_fb<Real>(a.R[lo], np, lo, a.dt, a.density, a.Xa, a.Da, a.Aa, fbl, tbl);
+    partner_fb<Real>(a.R[hi], np, hi, a.dt, a.density, a.Xa, a.Da, a.Aa, fbh, tbh);
+    V3d xl = zero3<double>(), xh = zero3<double>(), dl = zero3<double>(), dh = zero3<double>(), al = zero3<double>(),
+        ah = zero3<double>(), hinb = zero3<double>();
+    double rl = 0.0, rh = 0.0;
+    pair_rev<M>(t, a.pp, inv_dt, a.density, fbl - fbh, tbl, tbh, mk(a.Hout[k], a.Hout[cap + k], a.Hout[2 * cap + k]),
+                xl, xh, dl, dh, al, ah, rl, rh, hinb, bp);
+    a.Hin[k] = hinb.x; a.Hin[cap + k] = hinb.y; a.Hin[2 * cap + k] = hinb.z;
+    st_share(a.PC + 2 * (size_t)kShare * k, xl, dl, al, rl);
+    st_share(a.PC + 2 * (size_t)kShare * k + kShare, xh, dh, ah, rh);
+    return true;
+}
+// A bound particle's walls: their VJP needs only the particle's force adjoints,
+// so it runs beside the pairs.  False, with nothing written, out of M's range.
+template <class M, typename Real>
+__device__ __forceinline__ bool adj_walls(const AdjPairs<Real>& a, uint i, LawBar& b) {
+    const long long np = a.np;
+    V3d fbi, tbi;
+    partner_fb<Real>(a.R[i], np, i, a.dt, a.density, a.Xa, a.Da, a.Aa, fbi, tbi);
+    V3d xw = zero3<double>(), dw = zero3<double>(), aw = zero3<double>(), hwb = zero3<double>();
+    double rw = 0.0;
+    if (wall_vjp<M>(a.hx, a.hy, ld3(a.tx, np, i), ld3(a.td, np, i), ldA<Real>(a.ta, np, i), (double)a.R[i], a.density,
+                    ld3(a.twh, np, i), a.pw, 1.0 / a.dt, fbi, tbi, ld3(a.Wb, np, i), xw, dw, aw, rw, hwb, b) == 2)
+        return false;
+    st3(a.Wb, np, i, hwb);
+    st_share(a.WS + (size_t)kShare * i, xw, dw, aw, rw);
+    return true;
+}
+template <typename Real>
+__global__ void __launch_bounds__(kAB, 2) k_adj_pairs(const __grid_constant__ AdjPairs<Real> a) {
+    __shared__ long long s_q[(kAC + 1) * kAB];   // items that touch, waiting for a thread
+    __shared__ uint s_n[kAC][kAB / 32];
+    const long long np = a.np, cap = a.cap;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    LawBar bp;   // of the pairs, or of the walls
+    lawbar_zero(bp);
+    // the list and the tape (the recompute's) may be read before the wait;
+    // the state and history adjoints are the predecessors'
+    const uint total = a.L.off[a.n];
+    const long long nb = (long long)*a.nb;
+    const long long npr = (long long)total <= cap ? (long long)total : 0ll;
+    if (a.earlier) {   // the tape of the step before this one
+        prefetch_range(a.tx - 3 * np, 3 * np);
+        prefetch_range(a.td - 3 * np, 3 * np);
+        prefetch_range(a.ta - 3 * np, 3 * np);
+        prefetch_range(a.twh - 3 * np, 3 * np);
+        prefetch_range(a.tF - 3 * np, 3 * np);
+        prefetch_range(a.tT - 3 * np, 3 * np);
+        prefetch_range(a.tc - np, np);
+        for (int c = 0; c < 3; c++) prefetch_range(a.th - 3 * cap + c * cap, npr);
+    }
+    pdl_wait();
+    pdl_trigger();
+    // a sixteenth of the blocks take the particles' walls (few of which touch),
+    // the others the pairs, a contiguous run of them each
+    const unsigned wb = (gridDim.x + 15) / 16, pb = gridDim.x - wb;
+    if (blockIdx.x >= pb) {
+        for (long long u = (long long)(blockIdx.x - pb) * kAB + threadIdx.x; u < nb; u += (long long)wb * kAB) {
+            const uint i = a.blist[u];
+            double dl[5];
+            if (wall_prim(a.hx, a.hy, ld3(a.tx, np, i), (double)a.R[i], dl) >= 0) {
+                LawBar one;
+                lawbar_zero(one);
+                if (!adj_walls<MathFast, Real>(a, i, one)) {
+                    lawbar_zero(one);
+                    adj_walls<MathLib, Real>(a, i, one);
+                }
+                bp.estar += one.estar; bp.mu += one.mu; bp.cn += one.cn;
+                bp.ct += one.ct; bp.roll += one.roll; bp.roll_rel += one.roll_rel;
+            } else {
+                st3(a.Wb, np, i, zero3<double>());
+                no_share(a.WS + (size_t)kShare * i);
+            }
+        }
+        const double vw[6] = {bp.estar, bp.mu, bp.cn, bp.ct, bp.roll, bp.roll_rel};
+        block_sum6(vw, a.pbar + (size_t)blockIdx.x * 12 + 6);
+        return;
+    }
+    const long long per = (npr + pb - 1) / pb, first = (long long)blockIdx.x * per;
+    const long long last = first + per < npr ? first + per : npr;
+    uint waiting = 0;   // the same in every thread
+    for (long long c0 = first; c0 < last; c0 += kAC * kAB) {
+        bool on[kAC];
+#pragma unroll
+        for (int e = 0; e < kAC; e++) {
+            const long long k = c0 + e * kAB + threadIdx.x;
+            on[e] = false;
+            if (k < last) {
+                const uint lo = a.L.lp[k], hi = a.L.ln[k];
+                const uint cl = a.tc[lo], ch = a.tc[hi];
+                const V3d D = ld3(a.tx, np, hi) - ld3(a.tx, np, lo);
+                const double dist = sqrt(dot(D, D));
+                on[e] = cl != 0 && ch != 0 && ((double)a.R[lo] + (double)a.R[hi]) - dist > 0.0 && dist > 0.0;
+            }
+        }
+        uint m[kAC];
+#pragma unroll
+        for (int e = 0; e < kAC; e++) {
+            m[e] = __ballot_sync(0xffffffffu, on[e]);
+            if (lane == 0) s_n[e][warp] = __popc(m[e]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < kAC; e++) {
+            const long long k = c0 + e * kAB + threadIdx.x;
+            uint at = waiting + __popc(m[e] & ((1u << lane) - 1u));
+            for (int w = 0; w < kAB / 32; w++) {
+                if (w < warp) at += s_n[e][w];
+                waiting += s_n[e][w];
+            }
+            if (on[e]) {
+                s_q[at] = k;
+            } else if (k < last) {
+                a.Hin[k] = 0.0; a.Hin[cap + k] = 0.0; a.Hin[2 * cap + k] = 0.0;
+                no_share(a.PC + 2 * (size_t)kShare * k);
+                no_share(a.PC + 2 * (size_t)kShare * k + kShare);
+            }
+        }
+        __syncthreads();
+        const bool end = c0 + kAC * kAB >= last;
+        while (waiting >= (uint)kAB || (end && waiting > 0)) {
+            const uint take = waiting < (uint)kAB ? waiting : (uint)kAB;
+            waiting -= take;
+            if (threadIdx.x >= take) continue;
+            const long long item = s_q[waiting + threadIdx.x];
+            if (!adj_pair<MathFast, Real>(a, item, bp)) adj_pair<MathLib, Real>(a, item, bp);
+        }
+        __syncthreads();   // the queue's entries have been read
+    }
+    const double v[6] = {bp.estar, bp.mu, bp.cn, bp.ct, bp.roll, bp.roll_rel};
+    block_sum6(v, a.pbar + (size_t)blockIdx.x * 12);
 }
 
 template <typename Real>
 __global__ void __launch_bounds__(kAB) k_adj_bound(
     long long n, long long np, long long cap, AdjList L, const uint* __restrict__ blist, const uint* __restrict__ nbp,
     const double* __restrict__ tF, const double* __restrict__ tT, const Real* __restrict__ R, double dt,
-    double density, const double* __restrict__ PC, const uint* __restrict__ pon, const double* __restrict__ WS,
-    const uint* __restrict__ wson, const double* __restrict__ Xa, const double* __restrict__ Da,
-    const double* __restrict__ Aa, double* __restrict__ Xo, double* __restrict__ Do, double* __restrict__ Ao,
-    double* __restrict__ Rb) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    double density, const double* __restrict__ PC, const double* __restrict__ WS, const double* __restrict__ Xa,
+    const double* __restrict__ Da, const double* __restrict__ Aa, double* __restrict__ Xo, double* __restrict__ Do,
+    double* __restrict__ Ao, double* __restrict__ Rb) {
+    const long long stride = (long long)gridDim.x * (kAB / kBG);
+    long long u = (long long)blockIdx.x * (kAB / kBG) + threadIdx.x / kBG;
+    const uint sub = threadIdx.x % kBG;
     const long long nb = (long long)*nbp;
     const uint total = L.off[n];
     // the list and the tape of a particle (the first one before the wait)
@@ -665,26 +786,42 @@ __global__ void __launch_bounds__(kAB) k_adj_bound(
     if (u < nb) load();
     pdl_wait();
     pdl_trigger();
-    for (bool first = true; u < nb; u += stride, first = false) {
-        if (!first) load();
-        const V3d xa = ld3(Xa, np, i), aa = ld3(Aa, np, i);
-        V3d dtot, fbi, tbi;
+    for (bool again = false; __any_sync(0xffffffffu, u < nb); u += stride, again = true) {
+        const bool live = u < nb;
+        if (again && live) load();
+        V3d xb = zero3<double>(), dbv = zero3<double>(), ab = zero3<double>(), xa = xb, aa = xb, dtot = xb;
         double rb = 0.0;
-        integ_rev<Real>(rr, fi, ti, dt, density, xa, ld3(Da, np, i), aa, dtot, fbi, tbi, rb);
-        V3d xb = zero3<double>(), dbv = zero3<double>(), ab = zero3<double>();
-        if ((long long)total <= cap) {
-            for (uint k = o0; k < o1; k++)
-                if (pon[k]) add_share(PC + (size_t)kPC * k, xb, dbv, ab, rb);
-            for (uint q = q0; q < q1; q++) {
-                const uint k = L.rk[q];
-                if (k < total && pon[k]) add_share(PC + (size_t)kPC * k + 10, xb, dbv, ab, rb);
+        if (live) {
+            if (sub == 0) {
+                V3d fbi, tbi;
+                xa = ld3(Xa, np, i);
+                aa = ld3(Aa, np, i);
+                integ_rev<Real>(rr, fi, ti, dt, density, xa, ld3(Da, np, i), aa, dtot, fbi, tbi, rb);
+                add_share(WS + (size_t)kShare * i, xb, dbv, ab, rb);   // its walls (the pair phase's items)
+            }
+            if ((long long)total <= cap) {
+                const uint own = o1 - o0, all = own + (q1 - q0);
+                for (uint e = sub; e < all; e += kBG) {
+                    if (e < own) {
+                        add_share(PC + 2 * (size_t)kShare * (o0 + e), xb, dbv, ab, rb);
+                    } else {
+                        const uint k = L.rk[q0 + (e - own)];
+                        if (k < total) add_share(PC + 2 * (size_t)kShare * k + kShare, xb, dbv, ab, rb);
+                    }
+                }
             }
         }
-        if (wson[i]) add_share(WS + 10 * (size_t)i, xb, dbv, ab, rb);   // its walls (the pair phase's items)
-        st3(Xo, np, i, xa + xb);
-        st3(Do, np, i, dtot + dbv);
-        st3(Ao, np, i, aa + ab);
-        Rb[i] += rb;
+        double v[10] = {xb.x, xb.y, xb.z, dbv.x, dbv.y, dbv.z, ab.x, ab.y, ab.z, rb};
+#pragma unroll
+        for (int c = 0; c < 10; c++)
+#pragma unroll
+            for (int o = kBG / 2; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+        if (live && sub == 0) {
+            st3(Xo, np, i, xa + mk(v[0], v[1], v[2]));
+            st3(Do, np, i, dtot + mk(v[3], v[4], v[5]));
+            st3(Ao, np, i, aa + mk(v[6], v[7], v[8]));
+            Rb[i] += v[9];
+        }
     }
 }
 
@@ -704,7 +841,7 @@ int adj_grids(dem_ctx* c) {
         e = mx ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bb, k_adj_bound<float>, kAB, 0)
                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bb, k_adj_bound<double>, kAB, 0);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint kernel set-up", __FILE__, __LINE__);
-    w->grid_pairs = (unsigned)std::max(1, nsm * std::max(bp, 1));
+    w->grid_pairs = (unsigned)std::max(2, nsm * std::max(bp, 1));   // pairs and walls
     w->grid_bound = (unsigned)std::max(1, nsm * std::max(bb, 1));
     return DEM_OK;
 }
@@ -876,20 +1013,27 @@ template <typename Real> int adj_step(dem_ctx* c, long long t, const ListRec& l,
         // both phases programmatic: each waits for its predecessor before it
         // reads an adjoint (tape and list loads overlap the predecessor's tail)
         const bool pdl = c->pdl;
-        const double* tx = w->tx + 3 * np * t;
-        const double* td = w->td + 3 * np * t;
-        const Real* ta = (const Real*)w->ta + 3 * np * t;
-        DEM_CUDA_TRY(launch_ex(k_adj_pairs<Real>, w->grid_pairs, kAB, w->rs, pdl, c->n, np, cap, L, tx, td, ta,
-                               (const double*)w->th + 3 * cap * t, (const uint*)w->tc + np * t, (const Real*)c->rad,
-                               make_law<double>(c->mat.pp), c->cfg.dt, c->cfg.density, (const double*)w->Hb[hb],
-                               w->Hb[1 - hb], (const double*)w->Xb2[in], (const double*)w->Db2[in],
-                               (const double*)w->Ab2[in], w->PC, w->pon, w->pbar, l.blist, l.nb,
-                               (const double*)w->twh + 3 * np * t, make_law<double>(c->mat.pw), c->cfg.world[0] * 0.5,
-                               c->cfg.world[1] * 0.5, w->WS, w->wson, w->Wb));
+        AdjPairs<Real> p;
+        p.n = c->n; p.np = np; p.cap = cap;
+        p.L = L;
+        p.tx = w->tx + 3 * np * t; p.td = w->td + 3 * np * t;
+        p.ta = (const Real*)w->ta + 3 * np * t;
+        p.th = w->th + 3 * cap * t;
+        p.tc = w->tc + np * t;
+        p.R = (const Real*)c->rad;
+        p.pp = make_law<double>(c->mat.pp); p.pw = make_law<double>(c->mat.pw);
+        p.dt = c->cfg.dt; p.density = c->cfg.density; p.hx = c->cfg.world[0] * 0.5; p.hy = c->cfg.world[1] * 0.5;
+        p.Hout = w->Hb[hb]; p.Hin = w->Hb[1 - hb];
+        p.Xa = w->Xb2[in]; p.Da = w->Db2[in]; p.Aa = w->Ab2[in];
+        p.PC = w->PC; p.WS = w->WS; p.Wb = w->Wb; p.pbar = w->pbar;
+        p.blist = l.blist; p.nb = l.nb;
+        p.twh = w->twh + 3 * np * t; p.tF = w->tF + 3 * np * t; p.tT = w->tT + 3 * np * t;
+        p.earlier = t > 0;
+        DEM_CUDA_TRY(launch_ex(k_adj_pairs<Real>, w->grid_pairs, kAB, w->rs, pdl, p));
         DEM_CUDA_TRY(launch_ex(k_adj_bound<Real>, w->grid_bound, kAB, w->rs, pdl, c->n, np, cap, L, l.blist, l.nb,
                                (const double*)w->tF + 3 * np * t, (const double*)w->tT + 3 * np * t,
                                (const Real*)c->rad, c->cfg.dt, c->cfg.density, (const double*)w->PC,
-                               (const uint*)w->pon, (const double*)w->WS, (const uint*)w->wson,
+                               (const double*)w->WS,
                                (const double*)w->Xb2[in], (const double*)w->Db2[in], (const double*)w->Ab2[in],
                                w->Xb2[1 - in], w->Db2[1 - in], w->Ab2[1 - in], w->Rb));
         return DEM_OK;
@@ -1255,7 +1399,7 @@ extern "C" int dem_adjoint_release(dem_ctx* c) {
     for (Ck& k : w->ck) free_ck(k);
     if (w->rs) cudaStreamSynchronize(w->rs);
     void* p[] = {w->Xb2[0], w->Db2[0], w->Ab2[0], w->Xb2[1], w->Db2[1], w->Ab2[1], w->Wb, w->Rb, w->Hb[0], w->Hb[1],
-                 w->pbar, w->obj, w->zmax, w->save_mz, w->save_cnt, w->Pobj, w->objp, w->PC, w->pon, w->WS, w->wson};
+                 w->pbar, w->obj, w->zmax, w->save_mz, w->save_cnt, w->Pobj, w->objp, w->PC, w->WS};
     for (void* x : p)
         if (x) cudaFree(x);
     for (TapeSet& t : w->set) free_set(t);
