@@ -216,8 +216,9 @@ __device__ __forceinline__ uint curve_bin(const V3<double>& p, const GridC& g, c
 // and its particles' states in tile order.  One launch: as separate kernels
 // the window graph took 24 more nodes, 90 us longer to instantiate.  Bound by
 // the latency of its gathers; with the partners' slots held in registers and
-// three blocks per SM (85 registers): 44 -> 31 us for a bed of 20,000 spheres,
-// 88 -> 65 us of 100,000 in FP64, 187 -> 158 us of 500,000.
+// three blocks per SM (80 registers), and the plan made by every block instead of
+// behind a barrier: 44 -> 28 us for a bed of 20,000 spheres, 88 -> 62 us of
+// 100,000 in FP64, 187 -> 155 us of 500,000.
 template <typename Real, bool PP>
 __global__ void __launch_bounds__(TileCap<Real>::P, 3)
     k_tile_lists(StepArgs<Real> a, TileArgs<Real> T, const uint* __restrict__ bflag, GridC g, CurveGrid cg, uint ntmax,
@@ -236,31 +237,46 @@ __global__ void __launch_bounds__(TileCap<Real>::P, 3)
     const uint nbound = a.bpos[n];
     uint nbar = 0;
     for (uint t = gid; t < ntmax; t += nthr) T.flag[(size_t)t * kFlagStride] = 0u;
-    if (gid == 0) {
+    // the plan: every block makes it from the same words, the first writes it
+    // once all have read them (after the next barrier)
+    __shared__ uint s_plan[6];
+    if (p == 0) {
         const long long pairs = a.off[n];
         uint shrink = T.tw[kTwShrink];
-        if (T.tw[kTwOver] == 2u) T.tw[kTwShrink] = ++shrink;   // the last window's tiles did not fit
+        if (T.tw[kTwOver] == 2u) ++shrink;   // the last window's tiles did not fit
         TilePlan pl{0u, 0u};
         if (pairs <= a.cap)
             pl = tile_plan((long long)nbound, pairs, T.G, PC, TileCap<Real>::smem, (uint)sizeof(TileRec<Real>), RB, shrink);
         const uint nt = pl.p ? (nbound + pl.p - 1) / pl.p : 0u;
         const bool fits = nbound == 0u || (pl.p && nt <= ntmax);
-        T.tw[kTwP] = pl.p;
-        T.tw[kTwTiles] = nt;
-        T.tw[kTwStage] = pl.stage;
-        T.tw[kTwOver] = fits ? 0u : 1u;
         const uint age = T.tw[kTwAge];
-        const bool need = !T.tw[kTwValid] || age >= kCurveEvery;
-        T.tw[kTwNeed] = need && fits && nt ? 1u : 0u;
-        if (fits && nt) {
-            T.tw[kTwAge] = need ? 1u : age + 1u;
+        const bool need = (!T.tw[kTwValid] || age >= kCurveEvery) && fits && nt;
+        s_plan[0] = pl.p; s_plan[1] = nt; s_plan[2] = pl.stage; s_plan[3] = fits ? 0u : 1u;
+        s_plan[4] = need ? 1u : 0u;
+        s_plan[5] = shrink;
+    }
+    __syncthreads();
+    const uint PT = s_plan[0], nt = s_plan[1], stage = s_plan[2];
+    const bool go = PT != 0u && nt != 0u && nt <= ntmax;
+    auto barrier = [&]() { grid_barrier(bar, nbar++, gridDim.x, a.words); };
+    auto publish = [&]() {
+        if (gid != 0) return;
+        T.tw[kTwP] = PT;
+        T.tw[kTwTiles] = nt;
+        T.tw[kTwStage] = stage;
+        T.tw[kTwOver] = s_plan[3];
+        T.tw[kTwShrink] = s_plan[5];
+        if (go) {
+            T.tw[kTwAge] = s_plan[4] ? 1u : T.tw[kTwAge] + 1u;
             T.tw[kTwValid] = 1u;
         }
+    };
+    if (!go) {
+        barrier();
+        publish();
+        return;
     }
-    grid_barrier(bar, nbar++, gridDim.x, a.words);
-    const uint PT = __ldcg(T.tw + kTwP), nt = __ldcg(T.tw + kTwTiles), stage = __ldcg(T.tw + kTwStage);
-    if (PT == 0u || nt == 0u || nt > ntmax) return;
-    if (__ldcg(T.tw + kTwNeed)) {
+    if (s_plan[4]) {
         for (long long i = gid; i < n; i += nthr) {
             const uint c = curve_bin(ld_pos<false>(a.S + i), g, cg);
             key[i] = c;
@@ -310,6 +326,7 @@ __global__ void __launch_bounds__(TileCap<Real>::P, 3)
         uint* bs = bsum + gridDim.x;   // the curve's sums may still be read
         if (p == 0) bs[blockIdx.x] = mine;
         grid_barrier(bar, nbar++, gridDim.x, a.words);
+        publish();
         v = 0;
         for (uint k = p; k < blockIdx.x; k += kTileThreads) v += __ldcg(bs + k);
         s_own[p] = v;
