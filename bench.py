@@ -48,15 +48,26 @@ BYTES_PER_PAIR = 56                                 # ids 8 + FP64 history r+w 4
 METRIC = "particle-steps/s @500K spheres"
 UNIT = "particle-steps/s"
 def launches_per_window(work):
-    """Kernels a window graph launches when its outer candidate list stays
-    valid (a rebuild adds the 10 launches of the conditional node's body):
-    the outer check, the candidate pass with its scans, the fill, the reverse
-    rows, and with cluster batches the component pass; then the window
-    kernel, which with cluster batches exits unless a batch is too large, the
-    batches and the free particles."""
+    """Kernels a window launches in a context without tiles (no memory for
+    them) when its outer candidate list stays valid (a rebuild adds the 10
+    launches of the conditional node's body): the outer check, the candidate
+    pass with its scans, the fill, the reverse rows, and with cluster batches
+    the component pass; then the window kernel, which with cluster batches
+    exits unless a batch is too large, the batches and the free particles."""
     batching = work.get("batched", -1) >= 0
     relist = 4 + (1 if batching else 0)
     return relist + (3 if batching else 1)
+
+
+def launches_in_window(work):
+    """The same in a context with tiles: a window of batches launches the
+    batches and the free particles after the re-list; any other the tables,
+    the tiles and the grid-barrier kernel, which exits when the tiles fit,
+    beside them (batches and free particles: PCCP only)."""
+    batched = work.get("batched", -1)
+    if batched == 1:
+        return launches_per_window(work) - 1
+    return launches_per_window(work) + 2
 
 
 def load_pkg():
@@ -317,14 +328,14 @@ def run_ours(args):
                 "its DRAM traffic is far below this per-step byte model); the free ones run in registers "
                 "(k_free_run) on the second stream beside the re-list; latency-bound (block barriers)")
     elif kt["window_kernel_ms"] > 0:
-        kname, kms = "k_window", kt["window_kernel_ms"]
+        kname, kms = "k_tile_lists+k_tile", kt["window_kernel_ms"]
     else:   # per-step kernels
         kname, kms = "k_pair+k_particle", kt["pair_ms"] + kt["particle_ms"]
     head_roof = roofline(kname, kbytes, kms, peak, peak_kind, w.name,
                          traffic=profile_traffic(f"{kname.replace('+', '_')}_rsa500k_{args.precision}"), note=note)
     head_roof.update({"kernel_timing": "CUDA events inside the last timed window's graph; window_kernel_ms is the "
                                        "window's stepping (one launch of the window kernel, or the batched window: "
-                                       "its exiting window kernel and k_batch, joined with k_free_run, which the "
+                                       "k_batch, joined with k_free_run, which the "
                                        "re-list started) = the window's 20 steps, relist_ms one re-list",
                       "kernel_ms_all": kt, "window_work": work,
                       "step_bytes_per_window": kbytes + rbytes,
@@ -427,7 +438,7 @@ def run_ours(args):
                    "mean_cn": sc["mean_cn"]},
         "roofline": head_roof,
         "clocks": clk,
-        "gpu_launches": launches_per_window(work) * K,
+        "gpu_launches": launches_in_window(work) * K,
         "fp64_plain": fp64,
         "pp_mode": ppm,
         "settled_bed": bed,
@@ -493,8 +504,8 @@ def settled_bed(dem, torch, stream, flush, args, peak, peak_kind):
              "mean_cn": s["mean_cn"], "packing_fraction": s["packing_fraction"], "status": s["status"],
              "window_work": work, "kernel_ms": kt}
         if kt["window_kernel_ms"] > 0 and fm == dem.FORCE_PCCP:
-            r["roofline"] = roofline("k_window", kbytes, kt["window_kernel_ms"], peak, peak_kind, w.name,
-                                     traffic=profile_traffic(f"k_window_bed500k_{key}"),
+            r["roofline"] = roofline("k_tile_lists+k_tile", kbytes, kt["window_kernel_ms"], peak, peak_kind, w.name,
+                                     traffic=profile_traffic(f"k_tile_bed500k_{key}"),
                                      note="every sphere bound: B_p x 20 per sphere + 56 B x 20 per pair")
         r["step_achieved_gbs"] = (kbytes + rbytes) / (ms / kb / 1e3) / 1e9
         out[key] = r

@@ -325,9 +325,10 @@ int dem_window_kernel_times(dem_ctx* ctx, double out[5]);
  * pairs; the others step under gravity alone until the next re-list.
  * *batched = 1 when the bound particles' connected components (through the
  * pair list) were small enough to be stepped as cluster batches, one block
- * per batch in shared memory, 0 when the grid-barrier window kernel stepped
- * them (a dense bed is one large component), -1 when the context does not
- * batch (PP mode, DEM_B200_BATCH=0, per-step kernels).  Any pointer may be
+ * per batch in shared memory, 0 when they were stepped as tiles (a dense bed
+ * is one large component; the grid-barrier window kernel when a tile does not
+ * fit), -1 when the context does not batch (PP mode, DEM_B200_BATCH=0,
+ * per-step kernels).  Any pointer may be
  * NULL.  No
  * counterpart in the reference (it steps every particle the same way). */
 int dem_window_work(dem_ctx* ctx, long long* bound, long long* wall_candidates, long long* pairs, int* batched);
