@@ -907,7 +907,7 @@ __global__ void k_rev_sort(long long n, const uint* __restrict__ roff, uint* __r
 // resident block of k_batch where they fit (the batch window, cc_target),
 // that one block steps through the window in shared memory.  A batch above
 // the block's capacity (a bed of touching spheres is one component) sends
-// the whole window to the grid-barrier window kernel instead.
+// the whole window to the tiles (dem_tile.cuh) instead.
 
 // The batch window: the bound particles spread over the batch kernel's
 // resident blocks G, at least kBatchMin, at most P minus the largest component
@@ -986,7 +986,7 @@ __global__ void __launch_bounds__(kCcThreads)
         if (t < nb) {
             i = blist[t];
             r = parent[i];
-            if (r >= (uint)n || parent[r] != r) {   // not a root: the window goes to the grid-barrier kernel
+            if (r >= (uint)n || parent[r] != r) {   // not a root: the window goes to the tiles
                 atomicOr(ccw + 1, 1u);
                 r = kEmpty;
             } else if (r == i) {
@@ -1208,8 +1208,7 @@ __device__ __forceinline__ int pair_eval(V3<double> xi, V3<double> xj, V3<double
 // nonzero: a tile does not fit (the grid-barrier window kernel has the
 // window), [3] windows since the curve was computed, [4] nonzero: the curve
 // is valid, [5] bytes of a stage in shared memory, [6] sixteenths the tiles
-// are smaller because one did not fit, [7] nonzero: this window computes the
-// curve.
+// are smaller because one did not fit.
 enum : uint {
     kTwP = 0, kTwTiles = 1, kTwOver = 2, kTwAge = 3, kTwValid = 4, kTwStage = 5, kTwShrink = 6, kTwWords = 7
 };
@@ -1230,7 +1229,7 @@ template <typename Real> struct StepArgs {
     int split;                    // window kernels: bound items per thread of the bound blocks (0: all blocks)
     // cluster batches: when batch != 0 the window's bound particles are
     // stepped by k_batch unless ccw[1] (a component or batch too large) is
-    // set, in which case the grid-barrier window kernel steps the window
+    // set, in which case the tiles step the window
     int batch;
     const uint* ccw;
     const uint* tw;               // tile path's words (nullptr: no tiles)
@@ -1950,7 +1949,7 @@ template <typename Real>
 __global__ void __maxnreg__(BatchRegs<Real>::value) k_batch(StepArgs<Real> a, int K, const uint* __restrict__ corder,
                                                          const uint* __restrict__ cbatch, uint* cloc,
                                                          StepPartials part, size_t clr1) {
-    if (a.ccw[1]) return;   // a component or a batch too large: the grid-barrier window kernel has the window
+    if (a.ccw[1]) return;   // a component or a batch too large: the tiles have the window
     extern __shared__ __align__(16) unsigned char smem[];
     BatchSmem<Real> L;
     batch_smem_layout<Real>(smem, &L);
