@@ -3106,6 +3106,17 @@ int tiles_stale(dem_ctx* c) {
     return DEM_OK;
 }
 
+// What holds for the particles of the last re-list is void: their number or
+// places changed altogether (an upload, a layer that joins, a pour that is
+// set).  The outer list is rebuilt at the next re-list -- its rows name
+// particles by id, those no longer in the system among them, and have none
+// for the ones that came -- and so is the tiles' curve, an order of all of
+// them.
+int particles_changed(dem_ctx* c) {
+    DEM_CUDA_TRY(cudaMemsetAsync(c->oflag, 0x01, sizeof(uint), c->stream));
+    return tiles_stale(c);
+}
+
 // The next layer joins (dempacking.cu:459-461): nplayer more particles (the
 // rest at the end), and the step re-lists.
 int pour_insert(dem_ctx* c) {
@@ -3123,10 +3134,7 @@ int pour_insert(dem_ctx* c) {
     c->vol = 4.0 / 3.0 * M_PI * c->r3sum[nnew];
     c->in_window = 0;   // this step re-lists (m_hiall = 1)
     free_graphs(c);     // the particle count is part of every captured launch
-    if (const int rc = tiles_stale(c)) return rc;
-    // the new particles have no outer rows yet
-    DEM_CUDA_TRY(cudaMemsetAsync(c->oflag, 0x01, sizeof(uint), c->stream));
-    return DEM_OK;
+    return particles_changed(c);
 }
 
 size_t real_size(int prec) { return prec == DEM_PREC_MIXED ? sizeof(float) : sizeof(double); }
@@ -3571,9 +3579,7 @@ static int finish_upload(dem_ctx* c) {
     DEM_CUDA_TRY(cudaMemsetAsync(c->off[1], 0, (c->npad + 1) * sizeof(uint), c->stream));
     DEM_CUDA_TRY(cudaMemsetAsync(c->words, 0, sizeof(EngineWords), c->stream));
     if (c->cc_skip) DEM_CUDA_TRY(cudaMemsetAsync(c->cc_skip, 0, 2 * sizeof(uint), c->stream));
-    if (const int rc = tiles_stale(c)) return rc;
-    // the outer list is rebuilt at the first re-list (new positions, radii)
-    DEM_CUDA_TRY(cudaMemsetAsync(c->oflag, 0x01, sizeof(uint), c->stream));
+    if (const int rc = particles_changed(c)) return rc;   // new positions, radii
     DEM_CUDA_TRY(cudaMemsetAsync(c->lb, 0, lb_words(c->npad) * sizeof(uint), c->stream));
     DEM_CUDA_TRY(cudaMemsetAsync(c->part_mz, 0, (size_t)c->cfg.relist_interval * c->npart * sizeof(unsigned long long),
                                  c->stream));
@@ -3904,6 +3910,7 @@ int dem_set_pour(dem_ctx* c, long long nplayer, double tnewpar, long long n_acti
     for (long long i = 0; i < ntot; i++) c->r3sum[i + 1] = c->r3sum[i] + r[i] * r[i] * r[i];
     if (n_active != c->n) free_graphs(c);
     c->n = n_active;
+    if (const int rc = particles_changed(c)) return rc;
     c->vol = 4.0 / 3.0 * M_PI * c->r3sum[n_active];
     c->pour_nplayer = nplayer;
     c->pour_tnewpar = tnewpar;
