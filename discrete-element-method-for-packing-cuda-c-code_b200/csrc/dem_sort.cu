@@ -6,7 +6,8 @@
 // faster least significant digit radix sort for GPUs", 2022): tiles of 4,096
 // or 8,192 records take tickets, rank their records by digit (eight ballots in each
 // warp, in index order: stable; __match_any_sync took 3x as long), publish their digit counts, add up the
-// counts of the tiles before them (decoupled look-back, 16 tiles a round) and
+// counts of the tiles before them (decoupled look-back, 16 tiles a round; a
+// tile that waits too long for a count reads the records before it instead) and
 // write the records out from shared memory in digit order, so that the
 // writes are runs.  A pass reads and writes each record once.
 #include <mutex>
@@ -24,7 +25,11 @@ constexpr int kHistThreads = 256;
 // back over), of 256 x 16 below (50,000: 7.0 us, 512 x 16 9.3: more blocks).
 constexpr uint kRsLarge = 1u << 18;
 constexpr int kRsBack = 16;             // look-back words a thread loads side by side
-constexpr int kRsSpin = 1 << 22;        // polls of a word before the look-back gives up (it cannot: tickets)
+// Polls without a newly published word (~0.1 s) after which a tile no longer
+// waits and counts the records before it itself.  The tiles before it have all
+// started (tickets) and wait for none behind them, so this is for a block that
+// is kept from running: the order must not depend on how long that takes.
+constexpr int kRsSpin = 1 << 16;
 // scratch: digit counts of 4 passes, 4 tickets, then two regions of tiles x
 // 256 look-back words (a pass uses one and clears the other's for the next)
 constexpr size_t kRsHead = 4 * 256 + 64;
@@ -159,6 +164,7 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_pass(const uint2* __restri
     const uint first = rs_exscan<kRsWarps>(cnt, s_tmp);   // digit's first record in the sorted tile
     const uint global = rs_exscan<kRsWarps>(t < 256 ? hist[256 * pass + t] : 0u, s_tmp);   // and in the output
     W pre = 0;
+    bool gave_up = false;
     if (tile > 0 && t < 256) {
         long long b = (long long)tile - 1;
         int spin = 0;
@@ -177,16 +183,29 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_pass(const uint2* __restri
                 done = (w[k] & LbWord<W>::incl) != 0;
             }
             b -= used;
-            if (!used && ++spin > kRsSpin) break;
+            spin = used ? 0 : spin + 1;
+            gave_up = spin > kRsSpin;
+            if (gave_up) break;
         }
-        rs_store(mine, LbWord<W>::incl | (pre + (W)cnt));
+        if (!gave_up) rs_store(mine, LbWord<W>::incl | (pre + (W)cnt));
     }
     if (t < 256) {
         s_off[t] = global + (uint)pre - first;
 #pragma unroll
         for (int w = 0; w < kRsWarps; w++) s_cnt[w][t] += first;
     }
-    __syncthreads();
+    if (__syncthreads_or(gave_up)) {   // the records before this tile, counted from the input
+        uint* s_before = reinterpret_cast<uint*>(smem);
+        if (t < 256) s_before[t] = 0u;
+        __syncthreads();
+        for (uint j = t; j < base; j += kRsThreads) atomicAdd(&s_before[(in[j].x >> shift) & 255u], 1u);
+        __syncthreads();
+        if (gave_up) {
+            s_off[t] = global + s_before[t] - first;
+            rs_store(mine, LbWord<W>::incl | (W)(s_before[t] + cnt));
+        }
+        __syncthreads();
+    }
 #pragma unroll
     for (int e = 0; e < kRsItems; e++) {
         const uint j = warp * (kRsItems * 32) + e * 32 + lane;
