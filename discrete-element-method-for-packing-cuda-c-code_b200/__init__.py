@@ -98,6 +98,11 @@ class AdjointResult(ctypes.Structure):
                 ("adjoint_ms", ctypes.c_double)]
 
 
+class WindowInfo(ctypes.Structure):
+    _fields_ = [("path", ctypes.c_int), ("shrink", ctypes.c_int), ("tiles", ctypes.c_longlong),
+                ("tile_size", ctypes.c_longlong), ("blocks", ctypes.c_longlong)]
+
+
 class Deck(ctypes.Structure):
     _fields_ = [
         ("iforcemode", ctypes.c_int), ("ntot", ctypes.c_int),
@@ -167,6 +172,7 @@ _SIGS = [
     ("dem_kernel_times", ctypes.c_int, [_vp, _c_double_p]),
     ("dem_set_window_timing", ctypes.c_int, [_vp, ctypes.c_int]),
     ("dem_window_kernel_times", ctypes.c_int, [_vp, _c_double_p]),
+    ("dem_window_path", ctypes.c_int, [_vp, ctypes.POINTER(WindowInfo)]),
     ("dem_window_work", ctypes.c_int, [_vp, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong),
                                        ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_int)]),
     ("dem_adjoint_window", ctypes.c_int, [_vp, ctypes.c_longlong, ctypes.c_int, ctypes.c_int,
@@ -557,6 +563,14 @@ class Engine:
         check(lib().dem_window_work(self._h, ctypes.byref(b), ctypes.byref(w), ctypes.byref(p), ctypes.byref(bt)),
               "dem_window_work")
         return {"bound": b.value, "wall_candidates": w.value, "pairs": p.value, "batched": bt.value}
+
+    def window_path(self):
+        """How the bound particles of the last whole window were stepped:
+        "steps", "batches", "tiles" or "grid", and its tiles (dem_window_path)."""
+        w = WindowInfo()
+        check(lib().dem_window_path(self._h, ctypes.byref(w)), "dem_window_path")
+        return {"path": ("steps", "batches", "tiles", "grid")[w.path], "shrink": w.shrink, "tiles": w.tiles,
+                "tile_size": w.tile_size, "blocks": w.blocks}
 
     def window_kernel_times(self):
         out = (ctypes.c_double * 5)()

@@ -3079,6 +3079,7 @@ int launch_window_graph(dem_ctx* c) {
         if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate", __FILE__, __LINE__);
     }
     if (!direct) DEM_CUDA_TRY(cudaGraphLaunch(ge, c->stream));
+    c->window_ran = true;
     if (tm) c->wtiming_ran = true;
     const int K = c->cfg.relist_interval;
     c->hph = 0;
@@ -3592,6 +3593,7 @@ static int finish_upload(dem_ctx* c) {
     c->relists = 0;
     c->last_slot = -1;
     c->uploaded = true;
+    c->window_ran = false;
     return setup_grid(c);
 }
 
@@ -4308,6 +4310,29 @@ int dem_window_work(dem_ctx* c, long long* bound, long long* wall_candidates, lo
     if (wall_candidates) *wall_candidates = v[1];
     if (pairs) *pairs = (long long)v[2] <= c->cap ? v[2] : 0;
     if (batched) *batched = !use_batches(c) ? -1 : (v[3] == 0u ? 1 : 0);
+    return DEM_OK;
+}
+
+int dem_window_path(dem_ctx* c, dem_window_info* out) {
+    if (!c || !out) return fail(DEM_ERR_ARG, "dem_window_path: null argument");
+    memset(out, 0, sizeof(*out));
+    if (!c->uploaded || !c->window_ran || !c->win_kernel || c->record) return DEM_OK;
+    uint tw[kTwWords] = {}, dense = 1;
+    tw[kTwOver] = 1;
+    char* hp = (char*)c->host_pinned;
+    if (c->tw) DEM_CUDA_TRY(cudaMemcpyAsync(hp, c->tw, sizeof(tw), cudaMemcpyDeviceToHost, c->stream));
+    if (use_batches(c))
+        DEM_CUDA_TRY(cudaMemcpyAsync(hp + sizeof(tw), c->cc_words + 1, sizeof(uint), cudaMemcpyDeviceToHost, c->stream));
+    DEM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if (c->tw) memcpy(tw, hp, sizeof(tw));
+    if (use_batches(c)) memcpy(&dense, hp + sizeof(tw), sizeof(dense));
+    out->shrink = (int)tw[kTwShrink];
+    out->path = !dense ? DEM_WINDOW_BATCHES : tw[kTwOver] ? DEM_WINDOW_GRID : DEM_WINDOW_TILES;
+    if (out->path == DEM_WINDOW_TILES) {
+        out->tiles = tw[kTwTiles];
+        out->tile_size = tw[kTwP];
+        out->blocks = std::min<long long>(c->tile_grid, out->tiles);
+    }
     return DEM_OK;
 }
 

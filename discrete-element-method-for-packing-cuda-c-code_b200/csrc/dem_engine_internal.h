@@ -340,6 +340,7 @@ struct dem_ctx {
     unsigned tile_grid = 1, tile_list_grid = 1;
     uint* cbin = nullptr;            // the curve's bins: counts (ncbin), starts (ncbin), block sums
     uint ncbin = 0;
+    bool window_ran = false;         // a whole window has been launched since the upload
     bool window_follows = false;     // the re-list being enqueued is followed by a window (window_kernel)
     bool dense_cond = false;         // capturing: the tiles are a conditional node, switched by the component pass
     cudaGraphConditionalHandle dense_handle{};

@@ -332,6 +332,20 @@ int dem_window_kernel_times(dem_ctx* ctx, double out[5]);
  * NULL.  No
  * counterpart in the reference (it steps every particle the same way). */
 int dem_window_work(dem_ctx* ctx, long long* bound, long long* wall_candidates, long long* pairs, int* batched);
+/* How the bound particles of the last whole window were stepped (waits for
+ * the context's stream), the same state bit for bit either way. */
+#define DEM_WINDOW_STEPS   0   /* no whole window since the upload, or per-step kernels */
+#define DEM_WINDOW_BATCHES 1   /* cluster batches                                       */
+#define DEM_WINDOW_TILES   2   /* tiles                                                 */
+#define DEM_WINDOW_GRID    3   /* the grid-barrier window kernel                        */
+typedef struct {
+    int path;              /* DEM_WINDOW_*                                     */
+    int shrink;            /* sixteenths tiles are smaller, after some did not fit */
+    long long tiles;       /* tiles of the window (DEM_WINDOW_TILES, else 0)   */
+    long long tile_size;   /* particles per tile                               */
+    long long blocks;      /* blocks that step them                            */
+} dem_window_info;
+int dem_window_path(dem_ctx* ctx, dem_window_info* out);
 
 /* Checkpoint / resume (the reference's restart reader is commented out,
  * dempacking.cu:361-367, and its preflow.dat has no contact history).
