@@ -1208,9 +1208,11 @@ __device__ __forceinline__ int pair_eval(V3<double> xi, V3<double> xj, V3<double
 // nonzero: a tile does not fit (the grid-barrier window kernel has the
 // window), [3] windows since the curve was computed, [4] nonzero: the curve
 // is valid, [5] bytes of a stage in shared memory, [6] sixteenths the tiles
-// are smaller because one did not fit.
+// are smaller because one did not fit, [7] windows since that changed, [8]
+// windows for which no tiles are tried.  All zero after an upload.
 enum : uint {
-    kTwP = 0, kTwTiles = 1, kTwOver = 2, kTwAge = 3, kTwValid = 4, kTwStage = 5, kTwShrink = 6, kTwWords = 7
+    kTwP = 0, kTwTiles = 1, kTwOver = 2, kTwAge = 3, kTwValid = 4, kTwStage = 5, kTwShrink = 6, kTwSince = 7,
+    kTwRest = 8, kTwWords = 9
 };
 
 // Arguments of the PCCP step kernels (pair items, bound particles, free
@@ -3581,6 +3583,8 @@ static int finish_upload(dem_ctx* c) {
     DEM_CUDA_TRY(cudaMemsetAsync(c->words, 0, sizeof(EngineWords), c->stream));
     if (c->cc_skip) DEM_CUDA_TRY(cudaMemsetAsync(c->cc_skip, 0, 2 * sizeof(uint), c->stream));
     if (const int rc = particles_changed(c)) return rc;   // new positions, radii
+    // what the tiles of the state before needed says nothing about this one
+    if (c->tw) DEM_CUDA_TRY(cudaMemsetAsync(c->tw, 0, kTwWords * sizeof(uint), c->stream));
     DEM_CUDA_TRY(cudaMemsetAsync(c->lb, 0, lb_words(c->npad) * sizeof(uint), c->stream));
     DEM_CUDA_TRY(cudaMemsetAsync(c->part_mz, 0, (size_t)c->cfg.relist_interval * c->npart * sizeof(unsigned long long),
                                  c->stream));

@@ -56,6 +56,8 @@ constexpr uint kTileHash = 512;      // their hash set while they are collected
 constexpr uint kTileRow = 8;         // row entries that k_tile_lists holds in registers
 constexpr uint kFlagStride = 32;     // words between step counters: a 128-byte line each (in 14 shared lines the
                                      // polls of 436 tiles queued at a few L2 slices: ~4,800 cycles a wait)
+constexpr uint kTileRetry = 64;      // windows after which larger tiles are tried again (a window that does not fit
+                                     // costs its lists and the grid-barrier kernel's time: ~1 % if it fails again)
 constexpr uint kCurveEvery = 256;    // windows between two computations of the curve: at 0.1 m/s a sphere of the
                                      // 1 mm configurations moves 0.26 d in that time, so tiles stay compact
 
@@ -239,13 +241,24 @@ __global__ void __launch_bounds__(TileCap<Real>::P, 3)
     for (uint t = gid; t < ntmax; t += nthr) T.flag[(size_t)t * kFlagStride] = 0u;
     // the plan: every block makes it from the same words, the first writes it
     // once all have read them (after the next barrier)
-    __shared__ uint s_plan[6];
+    __shared__ uint s_plan[8];
     if (p == 0) {
         const long long pairs = a.off[n];
-        uint shrink = T.tw[kTwShrink];
-        if (T.tw[kTwOver] == 2u) ++shrink;   // the last window's tiles did not fit
+        // how much smaller: a sixteenth more after a window whose tiles did not
+        // fit, one less after kTileRetry windows; smaller tiles do not help one
+        // that has too many neighbours: no tiles for as many windows
+        const uint over = T.tw[kTwOver];
+        uint shrink = T.tw[kTwShrink], since = T.tw[kTwSince] + 1u, rest = T.tw[kTwRest];
+        if (over == 2u) {
+            ++shrink;
+            since = 0u;
+        } else if (shrink && since >= kTileRetry) {
+            --shrink;
+            since = 0u;
+        }
+        rest = over == 3u ? kTileRetry : rest ? rest - 1u : 0u;
         TilePlan pl{0u, 0u};
-        if (pairs <= a.cap)
+        if (pairs <= a.cap && !rest)
             pl = tile_plan((long long)nbound, pairs, T.G, PC, TileCap<Real>::smem, (uint)sizeof(TileRec<Real>), RB, shrink);
         const uint nt = pl.p ? (nbound + pl.p - 1) / pl.p : 0u;
         const bool fits = nbound == 0u || (pl.p && nt <= ntmax);
@@ -253,7 +266,7 @@ __global__ void __launch_bounds__(TileCap<Real>::P, 3)
         const bool need = (!T.tw[kTwValid] || age >= kCurveEvery) && fits && nt;
         s_plan[0] = pl.p; s_plan[1] = nt; s_plan[2] = pl.stage; s_plan[3] = fits ? 0u : 1u;
         s_plan[4] = need ? 1u : 0u;
-        s_plan[5] = shrink;
+        s_plan[5] = shrink; s_plan[6] = since; s_plan[7] = rest;
     }
     __syncthreads();
     const uint PT = s_plan[0], nt = s_plan[1], stage = s_plan[2];
@@ -266,6 +279,8 @@ __global__ void __launch_bounds__(TileCap<Real>::P, 3)
         T.tw[kTwStage] = stage;
         T.tw[kTwOver] = s_plan[3];
         T.tw[kTwShrink] = s_plan[5];
+        T.tw[kTwSince] = s_plan[6];
+        T.tw[kTwRest] = s_plan[7];
         if (go) {
             T.tw[kTwAge] = s_plan[4] ? 1u : T.tw[kTwAge] + 1u;
             T.tw[kTwValid] = 1u;
@@ -439,7 +454,7 @@ __global__ void __launch_bounds__(TileCap<Real>::P, 3)
                    nstage * stage + (tot + twall) * RB <= TileCap<Real>::smem;
         }
         if (!fits) {
-            if (p == 0) T.tw[kTwOver] = 2u;
+            if (p == 0) atomicMax(T.tw + kTwOver, nnbr > kTileNbr ? 3u : 2u);
             __syncthreads();   // s_nn is the next tile's
             continue;
         }

@@ -76,3 +76,40 @@ def test_long_row(dem, cuda, monkeypatch, prec, mode):
     assert e.window_path()["path"] == "tiles" and e.scalars()["max_row"] > 96
     e.close()
     check(dem, w, prec, monkeypatch, steps=60, mode=mode)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_an_upload_starts_over(dem, wl, cuda, prec, mode):
+    """A state whose tiles do not fit, then an even one in the same context:
+    its tiles are those of a new context from the first window on."""
+    even = dense_lattice(dem, 44, 44, 40)
+    uneven = crystal(dem, wl, 14, 14, 12, loose=(even.n - 14 * 14 * 12 * 4) // 2)
+    assert uneven.n == even.n
+    even.world = tuple(max(a, b) for a, b in zip(even.world, uneven.world))
+    uneven.world = even.world
+    new = engine(dem, even, prec, mode)
+    new.step(20)
+    used = engine(dem, uneven, prec, mode)
+    used.step(100)
+    assert used.window_path()["path"] == "grid" and used.window_path()["shrink"] > 1
+    used.upload(even.pos, even.rad)
+    used.step(20)
+    p = used.window_path()
+    assert p == new.window_path() and p["path"] == "tiles" and p["shrink"] == 0
+    for x, y in zip(new.download(), used.download()):
+        np.testing.assert_array_equal(x, y)
+    new.close()
+    used.close()
+
+
+def test_larger_tiles_are_tried_again(dem, wl, cuda):
+    """In one run: the shrink that a window left is lowered after a number of
+    windows, not kept for good."""
+    e = engine(dem, crystal(dem, wl, 14, 14, 12, loose=30000), 0, K=2)
+    seen = []
+    for _ in range(260):
+        e.step(2)
+        seen.append(e.window_path()["shrink"])
+    e.close()
+    assert max(seen) > 0 and any(b < a for a, b in zip(seen, seen[1:])), seen
