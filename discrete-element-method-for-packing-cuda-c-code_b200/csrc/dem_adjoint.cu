@@ -178,23 +178,23 @@ int ensure_work(dem_ctx* c, long long seg, long long nck) {
     const int K = c->cfg.relist_interval;
     int rc;
     if (!w->Xb) {
-        if ((rc = dalloc(&w->Xb2[0], 3 * np)) || (rc = dalloc(&w->Db2[0], 3 * np)) ||
-            (rc = dalloc(&w->Ab2[0], 3 * np)) || (rc = dalloc(&w->Xb2[1], 3 * np)) ||
-            (rc = dalloc(&w->Db2[1], 3 * np)) || (rc = dalloc(&w->Ab2[1], 3 * np)) || (rc = dalloc(&w->Wb, 3 * np)) ||
-            (rc = dalloc(&w->Rb, np)) || (rc = dalloc(&w->Hb[0], 3 * cap)) || (rc = dalloc(&w->Hb[1], 3 * cap)) ||
-            (rc = dalloc(&w->obj, 16)) ||
-            (rc = dalloc(&w->objp, 3 * (size_t)grid_for(c->n, kB))) ||
-            (rc = dalloc(&w->zmax, 2)) ||
-            (rc = dalloc(&w->save_mz, c->npart)) || (rc = dalloc(&w->save_cnt, c->npart)) ||
-            (rc = dalloc(&w->Pobj, 3 * np)))
+        if ((rc = dalloc(c, &w->Xb2[0], 3 * np)) || (rc = dalloc(c, &w->Db2[0], 3 * np)) ||
+            (rc = dalloc(c, &w->Ab2[0], 3 * np)) || (rc = dalloc(c, &w->Xb2[1], 3 * np)) ||
+            (rc = dalloc(c, &w->Db2[1], 3 * np)) || (rc = dalloc(c, &w->Ab2[1], 3 * np)) || (rc = dalloc(c, &w->Wb, 3 * np)) ||
+            (rc = dalloc(c, &w->Rb, np)) || (rc = dalloc(c, &w->Hb[0], 3 * cap)) || (rc = dalloc(c, &w->Hb[1], 3 * cap)) ||
+            (rc = dalloc(c, &w->obj, 16)) ||
+            (rc = dalloc(c, &w->objp, 3 * (size_t)grid_for(c->n, kB))) ||
+            (rc = dalloc(c, &w->zmax, 2)) ||
+            (rc = dalloc(c, &w->save_mz, c->npart)) || (rc = dalloc(c, &w->save_cnt, c->npart)) ||
+            (rc = dalloc(c, &w->Pobj, 3 * np)))
             return rc;
         const char* ap = getenv("DEM_B200_ADJ");   // "pp": the particle-parallel reverse step
         w->pair_parallel = !(ap && ap[0] == 'p');
         if ((rc = adj_grids(c))) return rc;
         w->npb = std::max<long long>(grid_for(c->n, kPairB), std::max(w->grid_pairs, w->grid_bound));
-        if ((rc = dalloc(&w->pbar, (size_t)w->npb * 12))) return rc;
-        if (w->pair_parallel && ((rc = dalloc(&w->PC, 2 * (size_t)kShare * cap)) ||
-                                 (rc = dalloc(&w->WS, kShare * (size_t)np))))
+        if ((rc = dalloc(c, &w->pbar, (size_t)w->npb * 12))) return rc;
+        if (w->pair_parallel && ((rc = dalloc(c, &w->PC, 2 * (size_t)kShare * cap)) ||
+                                 (rc = dalloc(c, &w->WS, kShare * (size_t)np))))
             return rc;
         w->Xb = w->Xb2[0];
         w->Db = w->Db2[0];
@@ -215,18 +215,18 @@ int ensure_work(dem_ctx* c, long long seg, long long nck) {
         const long long nw = (seg + K - 1) / K;
         for (TapeSet& t : w->set) {
             free_set(t);
-            if ((rc = dalloc(&t.tx, 3 * np * seg)) || (rc = dalloc(&t.td, 3 * np * seg)) ||
-                (rc = dalloc(&t.twh, 3 * np * seg)) || (rc = dalloc(&t.tF, 3 * np * seg)) ||
-                (rc = dalloc(&t.tT, 3 * np * seg)) || (rc = dalloc(&t.th, 3 * cap * seg)) ||
-                (rc = dalloc(&t.tc, np * seg)))
+            if ((rc = dalloc(c, &t.tx, 3 * np * seg)) || (rc = dalloc(c, &t.td, 3 * np * seg)) ||
+                (rc = dalloc(c, &t.twh, 3 * np * seg)) || (rc = dalloc(c, &t.tF, 3 * np * seg)) ||
+                (rc = dalloc(c, &t.tT, 3 * np * seg)) || (rc = dalloc(c, &t.th, 3 * cap * seg)) ||
+                (rc = dalloc(c, &t.tc, np * seg)))
                 return rc;
-            DEM_CUDA_TRY(cudaMalloc(&t.ta, 3 * np * seg * rsz(c)));
+            if ((rc = dalloc(c, (char**)&t.ta, 3 * np * seg * rsz(c)))) return rc;
             t.lists.resize(nw);
             for (ListRec& l : t.lists)
-                if ((rc = dalloc(&l.off, np + 1)) || (rc = dalloc(&l.ln, cap)) || (rc = dalloc(&l.lp, cap)) ||
-                    (rc = dalloc(&l.roff, np + 1)) || (rc = dalloc(&l.rk, cap)) || (rc = dalloc(&l.carry, cap)) ||
-                    (rc = dalloc(&l.bflag, np)) || (rc = dalloc(&l.blist, np)) || (rc = dalloc(&l.flist, np)) ||
-                    (rc = dalloc(&l.nb, 1)))
+                if ((rc = dalloc(c, &l.off, np + 1)) || (rc = dalloc(c, &l.ln, cap)) || (rc = dalloc(c, &l.lp, cap)) ||
+                    (rc = dalloc(c, &l.roff, np + 1)) || (rc = dalloc(c, &l.rk, cap)) || (rc = dalloc(c, &l.carry, cap)) ||
+                    (rc = dalloc(c, &l.bflag, np)) || (rc = dalloc(c, &l.blist, np)) || (rc = dalloc(c, &l.flist, np)) ||
+                    (rc = dalloc(c, &l.nb, 1)))
                     return rc;
         }
         w->seg = seg;
@@ -237,10 +237,10 @@ int ensure_work(dem_ctx* c, long long seg, long long nck) {
         w->ck.resize(nck);
         for (size_t k = old; k < (size_t)nck; k++) {
             Ck& x = w->ck[k];
-            if ((rc = dalloc(&x.q, np)) || (rc = dalloc(&x.wh, 3 * np)) || (rc = dalloc(&x.off, np + 1)) ||
-                (rc = dalloc(&x.ln, cap)) || (rc = dalloc(&x.hist, 3 * cap)))
+            if ((rc = dalloc(c, &x.q, np)) || (rc = dalloc(c, &x.wh, 3 * np)) || (rc = dalloc(c, &x.off, np + 1)) ||
+                (rc = dalloc(c, &x.ln, cap)) || (rc = dalloc(c, &x.hist, 3 * cap)))
                 return rc;
-            DEM_CUDA_TRY(cudaMalloc(&x.rec, np * recsz(c)));
+            if ((rc = dalloc(c, (char**)&x.rec, np * recsz(c)))) return rc;
         }
     }
     w->nck = nck;

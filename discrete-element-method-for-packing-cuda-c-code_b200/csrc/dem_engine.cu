@@ -22,6 +22,7 @@
 //    also reduces the observables (max height, contacts) on the device;
 //  * a whole re-list window (re-list + K steps) captured once as a CUDA graph;
 //    no host synchronisation inside dem_step_n.
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -955,7 +956,7 @@ __global__ void __launch_bounds__(kCcThreads)
               const uint* __restrict__ parent, const uint* __restrict__ size, const uint* __restrict__ pairs,
               uint* base, uint* __restrict__ fill, uint* __restrict__ order, uint* bw, uint* __restrict__ batch,
               uint* ccw, uint* __restrict__ cc_skip, uint* lbc, EngineWords* words, uint* bar, int cond,
-              cudaGraphConditionalHandle hw) {
+              cudaGraphConditionalHandle hw, volatile uint* seen) {
     constexpr int W = kCcThreads / 32;
     __shared__ uint s_tile, s_last, s_agg, s_pre;
     __shared__ uint s_w[W], s_red[W];
@@ -1111,7 +1112,19 @@ __global__ void __launch_bounds__(kCcThreads)
     }
     if (me < (uint)(2 * kBarWords)) bar[me] = 0u;   // the wait words of the kernels that follow
     __syncthreads();
-    if (cond && me == 0 && __ldcg(ccw + 1)) cudaGraphSetConditional(hw, 1u);   // the tiles' node
+    if (me == 0) {
+        const uint dense = __ldcg(ccw + 1);
+        if (cond && dense) cudaGraphSetConditional(hw, 1u);   // the tiles' node
+        // The host has not made the tiles yet: whether they are needed, or soon
+        // will be.  Told once each (a host write in every window is ~1 us).
+        const uint tell = !seen ? 0u : dense || maxc > P / 4 ? 2u : 1u;
+        if (tell > cc_skip[1]) {
+            cc_skip[1] = tell;
+            if (tell == 2u) seen[1] = 1u;
+            __threadfence_system();
+            seen[0] = 1u;
+        }
+    }
 }
 
 // ------------------------------------------------------------ pair force
@@ -2547,6 +2560,9 @@ template <typename Real> int outer_build_conditional(dem_ctx* c, const PRec<Real
 
 template <typename Real> int launch_free(dem_ctx* c, int lst, int slot0, int nsteps, cudaStream_t s, int batch = 0);
 
+// Whether the context has no tiles yet and may make them.
+bool tiles_pending(const dem_ctx* c) { return c->tiles_able && !c->tw; }
+
 template <typename Real> int launch_relist(dem_ctx* c, int src) {
     const long long n = c->n;
     const int dst = 1 - src;
@@ -2617,7 +2633,7 @@ template <typename Real> int launch_relist(dem_ctx* c, int src) {
                                (const uint*)c->blist, (const uint*)c->cc_parent, (const uint*)c->cc_size,
                                (const uint*)c->cc_pairs, c->cc_base, c->cc_fill, c->cc_order, c->cc_bw, c->cc_batch,
                                c->cc_words, c->cc_skip, c->lb + lb_cc(c->npad), c->words,
-                               c->bar, c->dense_cond ? 1 : 0, c->dense_handle));
+                               c->bar, c->dense_cond ? 1 : 0, c->dense_handle, tiles_pending(c) ? c->seen : nullptr));
     }
     return DEM_OK;
 }
@@ -2973,6 +2989,15 @@ int step_kernels(dem_ctx* c, int lst, int slot, double* ms_pair, double* ms_part
 }  // namespace dem
 
 namespace {
+int tiles_make(dem_ctx* c);
+
+// Waits (at most a second) until the component pass has told the host
+// whether its list needs tiles.
+void wait_seen(const dem_ctx* c) {
+    const auto t0 = std::chrono::steady_clock::now();
+    while (!c->seen[0] && std::chrono::steady_clock::now() - t0 < std::chrono::seconds(1)) {}
+}
+
 // Enqueue one full window (re-list from list `src`, then K steps).
 int enqueue_window(dem_ctx* c, int src) {
     const int K = c->cfg.relist_interval;
@@ -2984,6 +3009,10 @@ int enqueue_window(dem_ctx* c, int src) {
     c->window_follows = c->mode == DEM_FORCE_PCCP && !c->record && c->win_kernel && use_batches(c);
     int rc = relist(c, src);
     c->window_follows = false;
+    if (!rc && c->tiles_decide) {
+        wait_seen(c);
+        if (c->seen[1]) rc = tiles_make(c);
+    }
     if (rc) { c->free_early = false; return rc; }
     if (wt) DEM_CUDA_TRY(cudaEventRecordWithFlags(c->wev[1], c->stream, cudaEventRecordExternal));
     c->hph = 0;
@@ -3051,16 +3080,44 @@ bool window_direct(const dem_ctx* c) {
     return pour_due(c, c->step + (long long)kPourDirect * c->cfg.relist_interval - 1);
 }
 
+// Before a whole window of a context without tiles: makes them once a
+// component pass has asked for them.  Until then the host stays at most
+// 2 kTilesAhead windows ahead of the device, so that a gas that settles inside
+// one call gets its tiles as it does (an early sign, a component of a quarter
+// of a block, comes many windows before the first that needs them); the wait
+// gives up after 0.1 s, for a stream that waits for the caller.
+constexpr int kTilesAhead = 16;
+int tiles_check(dem_ctx* c) {
+    if (!c->seen[1] && ++c->ahead >= kTilesAhead) {
+        c->ahead = 0;
+        const auto t0 = std::chrono::steady_clock::now();
+        cudaError_t e;
+        while ((e = cudaEventQuery(c->evahead)) == cudaErrorNotReady &&
+               std::chrono::steady_clock::now() - t0 < std::chrono::milliseconds(100)) {}
+        if (e == cudaErrorNotReady) cudaGetLastError();
+        else if (e != cudaSuccess) return cuda_fail(e, "cudaEventQuery", __FILE__, __LINE__);
+        DEM_CUDA_TRY(cudaEventRecord(c->evahead, c->stream));
+    }
+    return c->seen[1] ? tiles_make(c) : DEM_OK;
+}
+
 // Launch a whole window for the current buffers: its graph, captured once, or
 // (window_direct) its kernels.
 int launch_window_graph(dem_ctx* c) {
     NvtxRange r("dem window graph");
+    const bool batched = use_batches(c) && c->win_kernel && !c->record;
+    if (batched && tiles_pending(c))
+        if (const int rc = tiles_check(c)) return rc;
     const int src = c->cur, sb = c->sbuf, hp = c->hph;
     const int tm = c->wtiming ? 1 : 0;
     cudaGraphExec_t& ge = c->gexec[src][sb][hp][tm];
-    const bool direct = !ge && window_direct(c);
+    // a new context's first window: its component pass says whether the
+    // graphs are captured with the tiles or without
+    c->tiles_decide = batched && tiles_pending(c) && !ge && !c->window_ran && !c->pouring && !tm;
+    const bool direct = !ge && (c->tiles_decide || window_direct(c));
     if (direct) {
         const int rc = enqueue_window(c, src);
+        c->tiles_decide = false;
         c->sbuf = sb;
         c->hph = hp;
         if (rc) return rc;
@@ -3156,12 +3213,12 @@ int host_perm(dem_ctx* c) {
 }
 }  // namespace dem
 
-// The tile path's arrays and launch shapes.  A context whose arrays do not
-// fit the device's memory goes without (c->tw stays null: such windows run
-// in the grid-barrier window kernel), as does one that re-lists every step
-// (the first and the last step of a window are then the same step, and a
-// pair across tiles would read a history that its owner writes).
-template <typename Real> int tiles_alloc(dem_ctx* c, cudaStream_t s) {
+namespace {
+// The tiles' launch shapes, set with the context: not able for a context that
+// re-lists every step (the first and the last step of a window are then the
+// same step, and a pair across tiles would read a history that its owner
+// writes).
+template <typename Real> int tiles_shape(dem_ctx* c) {
     int nsm = 0, per[2] = {0, 0};
     DEM_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     const size_t smem = TileCap<Real>::smem;
@@ -3174,24 +3231,55 @@ template <typename Real> int tiles_alloc(dem_ctx* c, cudaStream_t s) {
         DEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[k], fn[k], (int)TileCap<Real>::P, smem));
     }
     const int b = std::min(per[0], per[1]);
-    const long long np = c->npad;
     if (b < 1 || c->cfg.relist_interval < 2) return DEM_OK;
-    const uint G = (uint)(nsm * b);
-    const long long nt = tile_max(c->ntot, G, TileCap<Real>::floor);
-    const size_t Q = c->ntot <= (long long)G * TileCap<Real>::P ? TileCap<Real>::Q1 : TileCap<Real>::Q2;
-    c->tile_q = (uint)Q;
-    // the histories between the steps go into the per-pair results of the
-    // grid-barrier kernels, which a tiled window does not use, when they fit
-    const bool alias = !pp && (size_t)nt * Q * sizeof(double) <= (size_t)c->cap * 4 * real_size(c->prec);
-    double* own = nullptr;
-    c->tile_grid = (unsigned)std::min<long long>(G, nt);
     int lper = 0;
     DEM_CUDA_TRY(pp ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lper, k_tile_lists<Real, true>, (int)TileCap<Real>::P, 0)
                     : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lper, k_tile_lists<Real, false>,
                                                                     (int)TileCap<Real>::P, 0));
     if (lper < 1) return DEM_OK;
+    const uint G = (uint)(nsm * b);
+    const long long nt = tile_max(c->ntot, G, TileCap<Real>::floor);
+    c->tile_q = c->ntot <= (long long)G * TileCap<Real>::P ? TileCap<Real>::Q1 : TileCap<Real>::Q2;
+    c->tile_grid = (unsigned)std::min<long long>(G, nt);
     c->tile_list_grid = (unsigned)std::min<long long>((long long)std::min(lper, 4) * nsm, nt);
     c->ntile_max = nt;
+    c->tile_sms = nsm;
+    c->tiles_able = true;
+    return DEM_OK;
+}
+
+// The curve's bins for the context's world and largest radius: counts
+// (zeroed), starts, block sums.  DEM_ERR_CUDA when they do not fit.
+int tiles_bins(dem_ctx* c) {
+    const CurveGrid cg = curve_grid(c->cfg.world, 2.0 * c->rmax);
+    if (cg.nbins > c->ncbin) {
+        free_graphs(c);
+        if (c->cbin) {
+            DEM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+            cudaFree(c->cbin);
+            c->cbin = nullptr;
+            c->ncbin = 0;
+        }
+        const int rc = dalloc(&c->cbin, (size_t)2 * cg.nbins + (size_t)8 * c->tile_sms);
+        if (rc) return rc;
+        DEM_CUDA_TRY(cudaMemsetAsync(c->cbin, 0, (size_t)cg.nbins * sizeof(uint), c->stream));
+        c->ncbin = cg.nbins;
+    }
+    if (cg.cs != c->curve_cs) free_graphs(c);   // the cells' edge (r_max) is part of the captured launch
+    c->curve_cs = cg.cs;
+    return DEM_OK;
+}
+
+// The tiles' arrays.  A context whose arrays do not fit the device's memory
+// goes without from then on: such windows run in the grid-barrier kernel.
+template <typename Real> int tiles_alloc(dem_ctx* c) {
+    const bool pp = c->mode == DEM_FORCE_PP;
+    const long long np = c->npad, nt = c->ntile_max;
+    const size_t Q = c->tile_q;
+    // the histories between the steps go into the per-pair results of the
+    // grid-barrier kernels, which a tiled window does not use, when they fit
+    const bool alias = !pp && (size_t)nt * Q * sizeof(double) <= (size_t)c->cap * 4 * real_size(c->prec);
+    double* own = nullptr;
     struct Want { void** p; size_t bytes; };
     const Want want[] = {{(void**)&c->tw, kTwWords * sizeof(uint)},
                          {(void**)&c->tcurve, np * sizeof(uint)},
@@ -3205,12 +3293,13 @@ template <typename Real> int tiles_alloc(dem_ctx* c, cudaStream_t s) {
                          {(void**)&c->ts[1], np * sizeof(PRec<Real>)},
                          {(void**)&c->tq, np * sizeof(float4)},
                          {(void**)&own, alias ? 0 : nt * Q * 3 * sizeof(double)}};
-    // one allocation (each cudaMalloc costs the set-up ~0.1 ms)
+    // one allocation (each cudaMalloc costs ~0.1 ms)
     size_t total = 0;
     for (const Want& w : want) total += (w.bytes + 255) / 256 * 256;
-    if (cudaMalloc((void**)&c->tmem, total) != cudaSuccess) {
+    if (dalloc(&c->tmem, total)) {
         cudaGetLastError();   // out of memory: no tiles
         c->tmem = nullptr;
+        c->tiles_able = false;
         return DEM_OK;
     }
     size_t at = 0;
@@ -3223,14 +3312,39 @@ template <typename Real> int tiles_alloc(dem_ctx* c, cudaStream_t s) {
     } else {
         for (int k = 0; k < 3; k++) c->thist[k] = own + (size_t)k * nt * Q;
     }
-    DEM_CUDA_TRY(cudaMemsetAsync(c->tw, 0, kTwWords * sizeof(uint), s));
-    c->tile_sms = nsm;
+    DEM_CUDA_TRY(cudaMemsetAsync(c->tw, 0, kTwWords * sizeof(uint), c->stream));
+    if (c->uploaded && tiles_bins(c)) tiles_drop(c);
     return DEM_OK;
 }
 
-int tiles_create(dem_ctx* c, cudaStream_t s) {
-    return c->prec == DEM_PREC_MIXED ? tiles_alloc<float>(c, s) : tiles_alloc<double>(c, s);
+int tiles_make(dem_ctx* c) {
+    free_graphs(c);   // captured without them
+    return c->prec == DEM_PREC_MIXED ? tiles_alloc<float>(c) : tiles_alloc<double>(c);
 }
+}  // namespace
+
+namespace dem {
+bool tiles_drop(dem_ctx* c) {
+    if (!c->tmem) return false;
+    cudaDeviceSynchronize();   // the context's streams, the adjoint's among them
+    free_graphs(c);
+    cudaFree(c->tmem);
+    if (c->cbin) cudaFree(c->cbin);
+    cudaGetLastError();
+    c->tmem = nullptr;
+    c->cbin = nullptr;
+    c->ncbin = 0;
+    c->tw = c->tcurve = c->tinv = c->tflag = c->tk = nullptr;
+    c->thead = nullptr;
+    c->tblob = nullptr;
+    c->twl = nullptr;
+    c->ts[0] = c->ts[1] = nullptr;
+    c->tq = nullptr;
+    for (double*& h : c->thist) h = nullptr;
+    c->tiles_able = false;   // for good: the device is full
+    return true;
+}
+}  // namespace dem
 
 extern "C" {
 
@@ -3386,7 +3500,8 @@ int dem_create(const dem_config* cfg, dem_ctx** out) {
         }
     }
     // tiles: behind the cluster batches, and for every PP window
-    if ((c->batching || (c->mode == DEM_FORCE_PP && c->win_kernel)) && (rc = tiles_create(c, s0))) return bail(rc);
+    if (c->batching || (c->mode == DEM_FORCE_PP && c->win_kernel))
+        if ((rc = c->prec == DEM_PREC_MIXED ? tiles_shape<float>(c) : tiles_shape<double>(c))) return bail(rc);
     // partials per slot: the particle kernels' (at least as many as the
     // window kernels have blocks), then the free kernel's
     c->fpart = std::max<size_t>((size_t)c->nblk, std::max(c->win_grid, c->tile_grid));
@@ -3437,7 +3552,13 @@ int dem_create(const dem_config* cfg, dem_ctx** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->evdense, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->evdjoin, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->evahead, cudaEventDisableTiming);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate", __FILE__, __LINE__));
+    // PP windows run as tiles from the first one on; the batched mode's wait
+    // for the first window that needs them (tiles_check): a gas holds none
+    c->seen = (volatile uint*)((char*)c->host_pinned + 4032);
+    c->seen[0] = c->seen[1] = 0u;
+    if (c->mode == DEM_FORCE_PP && c->tiles_able && (rc = tiles_make(c))) return bail(rc);
     e = cudaStreamSynchronize(s0);   // the initialisation above is done
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamSynchronize", __FILE__, __LINE__));
     *out = c;
@@ -3476,6 +3597,7 @@ int dem_destroy(dem_ctx* c) {
     if (c->stream3) cudaStreamDestroy(c->stream3);
     if (c->evdense) cudaEventDestroy(c->evdense);
     if (c->evdjoin) cudaEventDestroy(c->evdjoin);
+    if (c->evahead) cudaEventDestroy(c->evahead);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
     return DEM_OK;
@@ -3536,7 +3658,7 @@ static int setup_grid(dem_ctx* c) {
         free_graphs(c);
         free_cells(c);
         int rc;
-        if ((rc = dalloc(&c->ccount, onc)) || (rc = dalloc(&c->cstart, onc + 1))) return rc;
+        if ((rc = dalloc(c, &c->ccount, onc)) || (rc = dalloc(c, &c->cstart, onc + 1))) return rc;
         DEM_CUDA_TRY(cudaMemsetAsync(c->ccount, 0, onc * sizeof(uint), c->stream));
         c->oncells = onc;
         size_t need = scan_scratch_words(std::max<long long>(onc, c->npad + 1));
@@ -3544,7 +3666,7 @@ static int setup_grid(dem_ctx* c) {
             DEM_CUDA_TRY(cudaStreamSynchronize(c->stream));
             cudaFree(c->scan_tmp);
             c->scan_tmp = nullptr;
-            if ((rc = dalloc(&c->scan_tmp, need))) return rc;
+            if ((rc = dalloc(c, &c->scan_tmp, need))) return rc;
             c->scan_words = need;
         }
     }
@@ -3555,24 +3677,7 @@ static int setup_grid(dem_ctx* c) {
     c->grid = g;
     c->ncells = nc;
     c->ogrid = og;
-    if (c->tw) {   // the tiles' curve bins: counts (zeroed), starts, block sums
-        const CurveGrid cg = curve_grid(c->cfg.world, 2.0 * c->rmax);
-        if (cg.nbins > c->ncbin) {
-            free_graphs(c);
-            if (c->cbin) {
-                DEM_CUDA_TRY(cudaStreamSynchronize(c->stream));
-                cudaFree(c->cbin);
-                c->cbin = nullptr;
-                c->ncbin = 0;
-            }
-            const int rc = dalloc(&c->cbin, (size_t)2 * cg.nbins + (size_t)8 * c->tile_sms);
-            if (rc) return rc;
-            DEM_CUDA_TRY(cudaMemsetAsync(c->cbin, 0, (size_t)cg.nbins * sizeof(uint), c->stream));
-            c->ncbin = cg.nbins;
-        }
-        if (cg.cs != c->curve_cs) free_graphs(c);   // the cells' edge (r_max) is part of the captured launch
-        c->curve_cs = cg.cs;
-    }
+    if (c->tw && tiles_bins(c)) tiles_drop(c);   // no room: without tiles
     return DEM_OK;
 }
 
@@ -3598,6 +3703,9 @@ static int finish_upload(dem_ctx* c) {
     c->last_slot = -1;
     c->uploaded = true;
     c->window_ran = false;
+    // no window of the state before is still at work (the upload waited for
+    // the stream)
+    c->seen[0] = c->seen[1] = 0u;
     return setup_grid(c);
 }
 
@@ -3646,8 +3754,8 @@ static int device_cell_order(dem_ctx* c, const double* pos, long long n, bool* o
     uint2* kv2 = kv + np;                            // 2 np words
     if (n < 65) return DEM_OK;   // fewer keep the caller's order
     int rc;
-    if (!c->perm && (rc = dalloc(&c->perm, np))) return rc;
-    if (!c->sort_tmp && (rc = dalloc(&c->sort_tmp, radix_scratch_words((uint)c->ntot)))) return rc;
+    if (!c->perm && (rc = dalloc(c, &c->perm, np))) return rc;
+    if (!c->sort_tmp && (rc = dalloc(c, &c->sort_tmp, radix_scratch_words((uint)c->ntot)))) return rc;
     k_cell_keys<<<grid_for(n, 256), 256, 0, c->stream>>>(n, pos, cs, 0.5 * c->cfg.world[0], 0.5 * c->cfg.world[1],
                                                          gx, gy, gz, kv);
     DEM_LAUNCH_CHECK();
@@ -3722,7 +3830,7 @@ static int upload_impl(dem_ctx* c, const double* pos, const double* pdis, const 
         } else if (order == kOrderGiven && given) {
             c->hperm.assign(given, given + n);
             if (!c->perm) {
-                int rc = dalloc(&c->perm, np);
+                int rc = dalloc(c, &c->perm, np);
                 if (rc) return rc;
             }
             DEM_CUDA_TRY(cudaMemcpyAsync(c->perm, c->hperm.data(), n * sizeof(uint), cudaMemcpyHostToDevice,
@@ -3896,7 +4004,8 @@ int dem_set_pour(dem_ctx* c, long long nplayer, double tnewpar, long long n_acti
         c->step = step;
         c->relists = relists;
     }
-    if (!c->pour_rec) DEM_CUDA_TRY(cudaMalloc(&c->pour_rec, (size_t)c->npad * recb));
+    if (!c->pour_rec)
+        if (const int rc = dalloc(c, (char**)&c->pour_rec, (size_t)c->npad * recb)) return rc;
     DEM_CUDA_TRY(cudaMemcpyAsync(c->pour_rec, c->rec[c->sbuf], (size_t)ntot * recb, cudaMemcpyDeviceToDevice, s));
     // r^3 prefix sums for the packing fraction of the particles in the system
     std::vector<double> r(ntot);
@@ -4093,8 +4202,8 @@ int dem_record_forces(dem_ctx* c, int on) {
     if (!c) return fail(DEM_ERR_ARG, "dem_record_forces: null ctx");
     if (on && !c->dbgF) {
         int rc;
-        if ((rc = dalloc(&c->dbgF, 3 * c->npad)) || (rc = dalloc(&c->dbgT, 3 * c->npad)) ||
-            (rc = dalloc(&c->dbgC, c->npad)))
+        if ((rc = dalloc(c, &c->dbgF, 3 * c->npad)) || (rc = dalloc(c, &c->dbgT, 3 * c->npad)) ||
+            (rc = dalloc(c, &c->dbgC, c->npad)))
             return rc;
     }
     if ((bool)on != c->record) free_graphs(c);

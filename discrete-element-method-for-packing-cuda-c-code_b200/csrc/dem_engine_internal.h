@@ -316,7 +316,7 @@ struct dem_ctx {
     uint* cc_order = nullptr;        // np: bound particle ids, grouped by component
     uint* cc_batch = nullptr;        // nbatch_max + 1: first slot of each batch
     uint* cc_loc = nullptr;          // np: a batch particle's index inside its block
-    uint* cc_skip = nullptr;         // [0] re-lists left that skip the component pass (a dense bed)
+    uint* cc_skip = nullptr;         // [0] re-lists left that skip the component pass (a dense bed), [1] what `seen` was told
     uint* cc_words = nullptr;        // [0] slots handed out, [1] 1 = a batch too large (or the list overflowed),
                                      // [2] largest component, [3] batch window (slots)
     long long nbatch_max = 0;
@@ -333,6 +333,14 @@ struct dem_ctx {
     float4* tq = nullptr;
     double* thist[3] = {nullptr, nullptr, nullptr};   // planes (pti, rfj and rtj, or thist_own)
     char* tmem = nullptr;            // the allocation that holds all of them
+    bool tiles_able = false;         // the launch shapes are set and the memory has not been refused or given back
+    // Pinned host words, written by the component pass while there are no
+    // tiles: [0] it has run since the upload, [1] a component was large enough
+    // that tiles will be needed (or are).
+    volatile uint* seen = nullptr;
+    bool tiles_decide = false;       // the window being launched waits for its component pass and decides
+    int ahead = 0;                   // windows launched since evahead was recorded
+    cudaEvent_t evahead = nullptr;
     int tile_sms = 0;
     double curve_cs = 0.0;           // edge of the curve's cells
     uint tile_q = 0;
@@ -425,5 +433,16 @@ template <typename T> int dalloc(T** p, size_t count) {
     if (count == 0) count = 1;
     DEM_CUDA_TRY(cudaMalloc((void**)p, count * sizeof(T)));
     return DEM_OK;
+}
+// Gives the tiles' memory back (the windows then run in the grid-barrier
+// kernel); false when there is none.
+bool tiles_drop(dem_ctx* c);
+// An allocation of a context at work: the tiles, which it can do without, make
+// room for it when the device is full.
+template <typename T> int dalloc(dem_ctx* c, T** p, size_t count) {
+    const int rc = dalloc(p, count);
+    if (!rc || !tiles_drop(c)) return rc;
+    cudaGetLastError();
+    return dalloc(p, count);
 }
 }  // namespace dem
