@@ -694,16 +694,26 @@ template <int N> __device__ __forceinline__ void sort_regs(uint (&r)[N]) {
                     }
 }
 
-// Whether the list is a bed's: many more pairs than a packing of small
-// components has, so that its particles are one large component and the
-// union-find would only find that out, with one root's counters added to by
-// every particle.  The 500,000-sphere gas has 0.51 pairs per bound particle, a
-// settled bed 3.5; below 5,120 pairs the components cost little.  The window
-// is then stepped as tiles, with the same bits.  Fill, reverse rows and
-// component pass of a 500,000-sphere bed's five re-lists after an upload: 1.52
-// + 1.65 + 1.11 ms before, 1.03 + 0.74 + 0.16 ms with this and the rows in
-// registers.
-__device__ __forceinline__ bool dense_list(long long pairs, long long nb) { return pairs > 5120 && 2 * pairs > 3 * nb; }
+// Whether the window's cluster batches cannot hold the list (their G resident
+// blocks; P particles and Q pairs each at most): a batch takes about
+// nb / G of the nb bound particles, at most P (an eighth less, for the largest
+// component, which is not known yet), and with the list's mean row that many
+// have more pairs than Q.  The union-find would only find that out -- in a
+// bed, which is one large component, with one root's counters added to by
+// every particle -- so no components are looked for, and the window is stepped
+// as tiles, with the same bits.  (A bed that is a small part of its system
+// passes; the component pass then finds its size and skips kDenseSkip windows.)
+// Fill, reverse rows and component pass of a 500,000-sphere bed's five re-lists
+// after an upload: 1.52 + 1.65 + 1.11 ms before, 1.03 + 0.74 + 0.16 ms with
+// this and the rows in registers.  Small dense components that fit stay with
+// the batches: five windows of 50,016 spheres, a fifth of them in clusters of
+// five (1.8 pairs each): 917 us as tiles, 667 as batches (mixed).
+struct BatchShape { uint G, P, Q; };
+__device__ __forceinline__ bool dense_list(long long pairs, long long nb, BatchShape s) {
+    const uint most = s.P - s.P / 8;
+    const long long t = max((long long)kBatchMin, min((nb + s.G - 1) / s.G, (long long)most));
+    return pairs * t > (long long)s.Q * nb;
+}
 
 // Fill the CSR row of i (j>i ascending), carry the FP64 tangential history
 // from the previous list, record the reverse slots.  Every particle with a
@@ -828,7 +838,7 @@ template <typename Real> __device__ __forceinline__ void fill_item(uint i, DEM_F
 // pass's look-back words (lbw of them) for the next re-list.
 template <typename Real>
 __global__ void __launch_bounds__(256, 4) k_nbr_fill(DEM_FILL_PARAMS, const uint* __restrict__ bpos, const uint* __restrict__ blist,
-                           const uint* __restrict__ cc_skip, uint* __restrict__ lb, long long lbw) {
+                           const uint* __restrict__ cc_skip, BatchShape bs, uint* __restrict__ lb, long long lbw) {
     pdl_wait();
     pdl_trigger();
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nthr = (long long)gridDim.x * blockDim.x;
@@ -838,7 +848,7 @@ __global__ void __launch_bounds__(256, 4) k_nbr_fill(DEM_FILL_PARAMS, const uint
         return;
     }
     const long long nb = bpos[n];
-    if (cc_parent && (*cc_skip || dense_list(off[n], nb))) cc_parent = nullptr;   // a bed: no components this re-list
+    if (cc_parent && (*cc_skip || dense_list(off[n], nb, bs))) cc_parent = nullptr;   // no components this re-list
     for (long long t = tid; t < nb; t += nthr) fill_item<Real>(blist[t], DEM_FILL_ARGS);
 }
 
@@ -865,12 +875,12 @@ __device__ __forceinline__ void rev_row(uint b, uint e, uint* __restrict__ rk, u
 __global__ void k_rev_sort(long long n, const uint* __restrict__ roff, uint* __restrict__ rk, uint* __restrict__ ru,
                            const uint* __restrict__ off, long long cap, uint* parent, const uint* __restrict__ bpos,
                            const uint* __restrict__ blist, uint* __restrict__ csize, uint* __restrict__ cpairs,
-                           const uint* __restrict__ cc_skip, uint* __restrict__ ccw) {
+                           const uint* __restrict__ cc_skip, BatchShape bs, uint* __restrict__ ccw) {
     pdl_wait();
     pdl_trigger();
     if ((long long)off[n] > cap) return;
     const long long nb = bpos[n];
-    if (parent && (*cc_skip || dense_list(off[n], nb))) parent = nullptr;
+    if (parent && (*cc_skip || dense_list(off[n], nb, bs))) parent = nullptr;
     uint mx = 0;   // the largest running component count: the largest component
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < nb;
          t += (long long)gridDim.x * blockDim.x) {
@@ -968,10 +978,10 @@ __global__ void __launch_bounds__(kCcThreads)
     const uint maxc = ccw[2];
     const bool over = (long long)off[n] > cap;
     const uint tgt = cc_target(nb, G, P, maxc);
-    // skip, or a bed's list: no components this re-list (the tiles have the
+    // skip, or a list too dense: no components this re-list (the tiles have the
     // window); every block still counts itself finished, and the last one
     // moves the skip count (cc_skip is read by every block first)
-    const bool run = !(skip || over || dense_list(off[n], nb));
+    const bool run = !(skip || over || dense_list(off[n], nb, BatchShape{G, P, Q}));
     if (!run && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(ccw + 1, 1u);
     if (run && blockIdx.x == 0 && threadIdx.x == 0) ccw[3] = tgt;
     const uint ntile = !run ? 0u : (nb == 0 ? 1u : (nb + kCcThreads - 1) / kCcThreads);
@@ -1101,10 +1111,6 @@ __global__ void __launch_bounds__(kCcThreads)
     }
     __syncthreads();
     if (!s_last) return;
-    if (me == 0) {
-        if (skip) *cc_skip = skip - 1u;
-        else if (maxc > P) *cc_skip = kDenseSkip;   // a component larger than a block (a dense bed)
-    }
     if (run && !__ldcg(ccw + 1)) {
         const uint nbatch = (nb + tgt - 1) / tgt;
         const uint bmax = (long long)nbatch < nbmax ? nbatch : (uint)nbmax;
@@ -1114,6 +1120,10 @@ __global__ void __launch_bounds__(kCcThreads)
     __syncthreads();
     if (me == 0) {
         const uint dense = __ldcg(ccw + 1);
+        if (skip) *cc_skip = skip - 1u;
+        // a component larger than a block (a dense bed), or batches that did
+        // not fit and are on average near what a block holds
+        else if (maxc > P || (run && dense && 5ll * off[n] * tgt > 4ll * Q * nb)) *cc_skip = kDenseSkip;
         if (cond && dense) cudaGraphSetConditional(hw, 1u);   // the tiles' node
         // The host has not made the tiles yet: whether they are needed, or soon
         // will be.  Told once each (a host write in every window is ~1 us).
@@ -2611,17 +2621,18 @@ template <typename Real> int launch_relist(dem_ctx* c, int src) {
     };
     if (c->free_early && c->free_fork == 1 && (rc = fork_free())) return rc;
     const unsigned BG = c->bound_grid;
+    const BatchShape bs{c->batch_grid, BatchCap<Real>::P, BatchCap<Real>::Q};
     DEM_CUDA_TRY(launch_ex(
         k_nbr_fill<Real>, BG, B, s, pdl, n, S, (const Real*)c->rad, g, skin, (const uint*)c->coff,
         (const uint*)c->cln, (const uint*)c->off[dst], (const uint*)c->roff,
         c->njli, c->ln[dst], c->lp, planes<double>(c->hist[dst][0], c->cap), (const uint*)c->off[src],
         (const uint*)c->ln[src], planes<double>(c->hist[src][c->hph], c->cap), c->rk, c->cap,
         c->words, c->carry, (const uint*)c->scr, cc ? c->cc_parent : nullptr, (const uint*)c->bpos,
-        (const uint*)c->blist, (const uint*)c->cc_skip, c->lb, (long long)lb_words(c->npad)));
+        (const uint*)c->blist, (const uint*)c->cc_skip, bs, c->lb, (long long)lb_words(c->npad)));
     if (c->free_early && c->free_fork == 2 && (rc = fork_free())) return rc;
     DEM_CUDA_TRY(launch_ex(k_rev_sort, BG, B, s, pdl, n, (const uint*)c->roff, c->rk, c->ru,
                            (const uint*)c->off[dst], c->cap, cc ? c->cc_parent : nullptr, (const uint*)c->bpos,
-                           (const uint*)c->blist, c->cc_size, c->cc_pairs, (const uint*)c->cc_skip, c->cc_words));
+                           (const uint*)c->blist, c->cc_size, c->cc_pairs, (const uint*)c->cc_skip, bs, c->cc_words));
     if (cc) {   // the window's components and batches (cluster-batched window path)
         c->dense_cond = graph && c->window_follows;
         c->dense_handle = cudaGraphConditionalHandle{};
