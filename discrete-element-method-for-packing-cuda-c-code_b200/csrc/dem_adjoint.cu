@@ -533,9 +533,12 @@ __global__ void __launch_bounds__(kPairB) k_adj_step(
 // touches: a law and its reverse are one chain of ~1,000 instructions, for
 // which a warp with half its lanes idle waits just as long.  The branch-free
 // quotients and roots (MathFast) shorten that chain; a pair out of their range
-// is done again with the library's.  A sixteenth of the blocks reverse the
-// bound particles' walls instead (slots 6-11, shares in WS): few particles
-// touch one, and among the pairs their chains were the last to end.
+// is done again with the library's.  Some of the blocks reverse the bound
+// particles' walls instead (slots 6-11, shares in WS): few particles touch one,
+// and among the pairs their chains were the last to end.  A sixteenth of the
+// blocks do beside a bed's pairs; where the pairs are few, a thread per
+// particle (50,000 spheres, 9,000 bound, 4,800 pairs, a reversed step: four
+// particles after one another in a sixteenth's threads 21.9 us, one 19.5 us).
 //
 // Phase B (k_adj_bound), kBG lanes per bound particle: the integrator reverse
 // and the sum of its pairs' shares (lane l the l-th, l+kBG-th ... of its own
@@ -679,9 +682,11 @@ __global__ void __launch_bounds__(kAB, 2) k_adj_pairs(const __grid_constant__ Ad
     }
     pdl_wait();
     pdl_trigger();
-    // a sixteenth of the blocks take the particles' walls (few of which touch),
-    // the others the pairs, a contiguous run of them each
-    const unsigned wb = (gridDim.x + 15) / 16, pb = gridDim.x - wb;
+    // some of the blocks take the particles' walls, the others the pairs, a
+    // contiguous run of them each: a sixteenth (few particles touch a wall), or
+    // a thread per particle where the pairs leave that many blocks
+    const long long wants = (nb + kAB - 1) / kAB, left = (long long)gridDim.x - (npr + kAB - 1) / kAB;
+    const unsigned wb = (unsigned)max((long long)(gridDim.x + 15) / 16, min(wants, left)), pb = gridDim.x - wb;
     if (blockIdx.x >= pb) {
         for (long long u = (long long)(blockIdx.x - pb) * kAB + threadIdx.x; u < nb; u += (long long)wb * kAB) {
             const uint i = a.blist[u];
