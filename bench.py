@@ -48,26 +48,23 @@ BYTES_PER_PAIR = 56                                 # ids 8 + FP64 history r+w 4
 METRIC = "particle-steps/s @500K spheres"
 UNIT = "particle-steps/s"
 def launches_per_window(work):
-    """Kernels a window launches in a context without tiles (no memory for
-    them) when its outer candidate list stays valid (a rebuild adds the 10
-    launches of the conditional node's body): the outer check, the candidate
-    pass with its scans, the fill, the reverse rows, and with cluster batches
-    the component pass; then the window kernel, which with cluster batches
-    exits unless a batch is too large, the batches and the free particles."""
+    """Kernels of a window that the grid-barrier kernel steps (a context that
+    was refused the memory of the tiles, a bed) when its outer candidate list
+    stays valid (a rebuild adds the 10 launches of the conditional node's
+    body): the outer check, the candidate pass with its scans, the fill, the
+    reverse rows, and with cluster batches the component pass; then the window
+    kernel, and with cluster batches these, which exit, and the free particles."""
     batching = work.get("batched", -1) >= 0
     relist = 4 + (1 if batching else 0)
     return relist + (3 if batching else 1)
 
 
 def launches_in_window(work):
-    """The same in a context with tiles: a window of batches launches the
-    batches and the free particles after the re-list; any other the tables,
-    the tiles and the grid-barrier kernel, which exits when the tiles fit,
-    beside them (batches and free particles: PCCP only)."""
-    batched = work.get("batched", -1)
-    if batched == 1:
-        return launches_per_window(work) - 1
-    return launches_per_window(work) + 2
+    """The same of a window of cluster batches (the re-list's five, the batches,
+    the free particles), of tiles (beside those: the tables, the tiles and the
+    grid-barrier kernel, which exits) and of a PP window (the re-list's four,
+    tables, tiles, window kernel, free particles)."""
+    return {1: 7, 0: 10}.get(work.get("batched", -1), 8)
 
 
 def load_pkg():

@@ -1393,7 +1393,7 @@ __global__ void __launch_bounds__(256) k_pair(StepArgs<Real> a) {
 
 // --------------------------------------------------- particle update
 // Per-step observables are written as one partial per block (no same-address
-// atomics in the hot kernels) and reduced on the host when asked for.
+// atomics in the hot kernels) and reduced by k_scalars when asked for.
 
 // One step of the integrator for one particle, in registers (updatepositionD,
 // neiglist.cu:356-360: symplectic Euler in displacement form), then the
@@ -3079,11 +3079,12 @@ int enqueue_window(dem_ctx* c, int src) {
 // A layer that joins drops the window graphs (the particle count is part of
 // every captured launch), and the two graphs of the next particle count cost
 // ~0.9 ms to capture and instantiate; a window launched directly costs ~0.1 ms
-// of host time and runs through the outer build's launches (~20 us more).  So while the next layer
-// is fewer than kPourDirect windows away, a small system's windows are
-// launched directly (above 2^16 particles the extra passes over them cost
-// more).  2,000 spheres, a call of 200 steps that ends before the next layer:
-// 2.30 ms with the graphs, 1.70 direct.
+// of host time and runs through the outer build's launches (~20 us more, and
+// passes over the particles that leave at once).  So while the next layer is
+// fewer than kPourDirect windows away, a small system's windows are launched
+// directly.  A call of 200 steps that ends before the next layer, graphs and
+// direct: 2,000 spheres 2.2 and 1.6 ms, 65,000 4.3 and 3.6, 200,000 7.9 and
+// 7.1, 400,000 13.6 and 18.9.
 bool pour_due(const dem_ctx* c, long long s);
 constexpr int kPourDirect = 16;
 bool window_direct(const dem_ctx* c) {

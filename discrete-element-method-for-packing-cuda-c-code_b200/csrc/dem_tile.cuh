@@ -105,8 +105,13 @@ template <typename Real> struct TileArgs {
 // memory of one stage (states and tables).  f pairs per particle; a fraction c ~ 1.45 /
 // P^(1/3) of a tile's pairs crosses its surface (a cube of P particles
 // loses 1.5 / P^(1/3)); 15 % of the pairs' bytes for uneven density, and
-// `shrink` sixteenths less after a window in which a tile did not fit.  One tile per
-// block when the system fits the resident blocks (its states then stay in
+// `shrink` sixteenths less after a window in which a tile did not fit.  A
+// stage that is the average tile's with the spare room shared out refuses a
+// dense core under a loose cloud at any size (rows of 6 among a mean of 1.2):
+// such windows stay with the grid-barrier kernel, which is the faster one
+// there in PCCP (stages as the largest tile needs let them run as tiles: 69,408
+// spheres FP64 414 -> 522 us a window, 246,080 mixed 716 -> 747; PP 988 -> 523
+// and 991 -> 744).  One tile per block when the system fits the resident blocks (its states then stay in
 // shared memory), else two stages per block (the next tile's loads run beside
 // the current one's steps), evened out over whole rounds of the G blocks.
 struct TilePlan { uint p, stage; };

@@ -84,9 +84,9 @@ int dem_compat_set_stream(void* cuda_stream);
 
 /* RadixSort(pData0, pData1, elements, keybits)  -- dempacking.cu:553-555.
  * Stable LSD sort of `elements` records by the low `keybits` bits of key;
- * result in pData0, pData1 is the ping-pong buffer.  Scratch for the digit
- * histograms is allocated by the library on the first call per device and
- * kept until exit. */
+ * result in pData0, pData1 is the ping-pong buffer.  Scratch (digit counts and
+ * look-back words) is allocated by the library on the first call per device
+ * and kept until exit. */
 int RadixSort(KeyValuePair* pData0, KeyValuePair* pData1,
               unsigned int elements, unsigned int keybits);
 
@@ -326,10 +326,9 @@ int dem_window_kernel_times(dem_ctx* ctx, double out[5]);
  * *batched = 1 when the bound particles' connected components (through the
  * pair list) were small enough to be stepped as cluster batches, one block
  * per batch in shared memory, 0 when they were stepped as tiles (a dense bed
- * is one large component; the grid-barrier window kernel when a tile does not
- * fit), -1 when the context does not batch (PP mode, DEM_B200_BATCH=0,
- * per-step kernels).  Any pointer may be
- * NULL.  No
+ * is one large component; the grid-barrier window kernel when the tiles do not
+ * fit: dem_window_path tells), -1 when the context does not batch (PP mode,
+ * DEM_B200_BATCH=0, per-step kernels).  Any pointer may be NULL.  No
  * counterpart in the reference (it steps every particle the same way). */
 int dem_window_work(dem_ctx* ctx, long long* bound, long long* wall_candidates, long long* pairs, int* batched);
 /* How the bound particles of the last whole window were stepped (waits for
