@@ -3338,7 +3338,7 @@ int tiles_make(dem_ctx* c) {
 namespace dem {
 bool tiles_drop(dem_ctx* c) {
     if (!c->tmem) return false;
-    cudaDeviceSynchronize();   // the context's streams, the adjoint's among them
+    cudaStreamSynchronize(c->stream);   // every window's branches join it; the adjoint's reverse stream has no use for them
     free_graphs(c);
     cudaFree(c->tmem);
     if (c->cbin) cudaFree(c->cbin);
