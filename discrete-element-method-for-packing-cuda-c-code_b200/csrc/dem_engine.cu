@@ -178,6 +178,17 @@ __global__ void k_pour_activate(long long nold, long long nnew, const PRec<Real>
     off[i + 1] = off[nold];
 }
 
+// A pour that is set on a context that has stepped: particles n and up leave
+// the system and will join anew, so the current list's pairs with them lose
+// their history (their own rows are emptied as they join).
+__global__ void k_pour_forget(long long n, long long cap, const uint* __restrict__ off, const uint* __restrict__ ln,
+                              Planes3<double> H) {
+    const long long np = off[n];
+    if (np > cap) return;
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < np; k += (long long)gridDim.x * blockDim.x)
+        if ((long long)ln[k] >= n) { H.x[k] = 0.0; H.y[k] = 0.0; H.z[k] = 0.0; }
+}
+
 // --------------------------------------------------------------- re-list
 // Outside a graph the outer build's kernels are launched at every re-list and
 // those that do the work leave at once when the check found the list still
@@ -4036,6 +4047,11 @@ int dem_set_pour(dem_ctx* c, long long nplayer, double tnewpar, long long n_acti
     c->r3sum.assign(ntot + 1, 0.0);
     for (long long i = 0; i < ntot; i++) c->r3sum[i + 1] = c->r3sum[i] + r[i] * r[i] * r[i];
     if (n_active != c->n) free_graphs(c);
+    if (n_active < c->n && c->relists) {
+        k_pour_forget<<<148, 256, 0, s>>>(n_active, c->cap, c->off[c->cur], c->ln[c->cur],
+                                          planes<double>(c->hist[c->cur][c->hph], c->cap));
+        DEM_LAUNCH_CHECK();
+    }
     c->n = n_active;
     if (const int rc = particles_changed(c)) return rc;
     c->vol = 4.0 / 3.0 * M_PI * c->r3sum[n_active];

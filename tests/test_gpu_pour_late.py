@@ -78,3 +78,35 @@ def test_layer_after_steps(dem, cuda, mode):
         e.close()
     for x, y in zip(*out):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_who_joins_again_has_no_history(dem, cuda, prec, mode):
+    """With friction: all the particles that a late pour took out join before
+    its first step, at the places they had, so their contacts with the others
+    are still listed -- and start without history, as in a new context."""
+    w = dense_lattice(dem, 14, 14, 12)
+    n_active = w.n // 2
+    out = []
+    a, b = (dem.Engine(**{**w.engine_kwargs(), "precision": prec, "force_mode": mode}) for _ in range(2))
+    zero = np.zeros(3 * w.n)
+    for e in (a, b):
+        e.set_material(w.pp, w.pw)
+    _upload(a, cuda, w, [w.pos, zero, zero], True)
+    a.step(40)
+    _upload(b, cuda, w, a.download(), True)
+    for e in (a, b):
+        e.set_pour(w.n - n_active, 1e-30, n_active)
+        e.step(1)
+        assert e.active_count() == w.n and e.scalars()["status"] == 0
+        lp, ln, h = e.pairs()
+        joined = ln >= n_active
+        out.append((lp, ln, np.asarray(h).reshape(-1, 3), joined))
+        e.close()
+    (lp, ln, h, joined), (lp2, ln2, h2, _) = out
+    np.testing.assert_array_equal(lp, lp2)
+    np.testing.assert_array_equal(ln, ln2)
+    assert joined.any() and (~joined).any() and np.abs(h2[joined]).max() > 0
+    np.testing.assert_array_equal(h[joined], h2[joined])
+    assert np.abs(h[~joined] - h2[~joined]).max() > 0   # the others kept theirs
